@@ -431,34 +431,43 @@ PyObject* gqa_decode_attention(PyObject* const* a)
     return wrap(std::move(out));
 }
 
+// A snapshot of any iterable as a tuple.  It owns its items, so that those of a sequence that makes them on
+// the fly (an array, a range) live as long as the call, and a list that another thread changes meanwhile
+// does not matter.
+struct items
+{
+    PyObject* tuple;
+    explicit items(PyObject* o) : tuple(PySequence_Tuple(o))
+    {
+        if(tuple == nullptr)
+            throw py_error{};
+    }
+    items(const items&) = delete;
+    items& operator=(const items&) = delete;
+    ~items() { Py_DECREF(tuple); }
+    Py_ssize_t size() const { return PyTuple_GET_SIZE(tuple); }
+    PyObject* operator[](Py_ssize_t i) const { return PyTuple_GET_ITEM(tuple, i); }
+};
+
 // (inputs, program, lens, op codes by name)
 PyObject* pointwise(PyObject* const* a)
 {
-    PyObject *ins = a[0], *prog = a[1], *lens = a[2], *ops = a[3];
-    if(not PySequence_Check(ins) or not PySequence_Check(prog) or not PySequence_Check(lens))
-        fail(PyExc_TypeError, "inputs, program and lens are sequences");
-    const auto ni = PySequence_Size(ins), np = PySequence_Size(prog), nd = PySequence_Size(lens);
+    const items ins(a[0]), prog(a[1]), lens(a[2]);
+    PyObject* ops = a[3];
+    const auto ni = ins.size(), np = prog.size(), nd = lens.size();
     if(ni < 1 or np < 1)
         fail(PyExc_IndexError, "at least one input and one instruction");
     if(ni > MGX_PW_MAXIN or np > MGX_PW_MAXINSN or nd > MGX_PW_MAXDIMS)
         fail(PyExc_IndexError, "too many inputs, instructions or dimensions");
-    auto item = [](PyObject* s, Py_ssize_t i) {
-        // kept alive by the sequence it came from (lists and tuples)
-        PyObject* o = PySequence_GetItem(s, i);
-        if(o == nullptr)
-            throw py_error{};
-        Py_DECREF(o);
-        return o;
-    };
     mgx_pw_desc d{};
     d.ndim = static_cast<int>(nd), d.ninputs = static_cast<int>(ni), d.ninsns = static_cast<int>(np);
     for(Py_ssize_t k = 0; k < nd; ++k)
-        d.lens[k] = integer(item(lens, k));
+        d.lens[k] = integer(lens[k]);
     const at::IntArrayRef sizes(d.lens, static_cast<size_t>(nd));
     const void* in[MGX_PW_MAXIN];
     for(Py_ssize_t i = 0; i < ni; ++i)
     {
-        const at::Tensor& t = tensor(item(ins, i));
+        const at::Tensor& t = tensor(ins[i]);
         if(t.sizes() != sizes)
             fail(PyExc_AssertionError, "an input does not have the shape of the result");
         d.in_type[i] = code_of(t.scalar_type());
@@ -468,19 +477,19 @@ PyObject* pointwise(PyObject* const* a)
     }
     for(Py_ssize_t n = 0; n < np; ++n)
     {
-        PyObject* t = item(prog, n);
-        if(not PySequence_Check(t) or PySequence_Size(t) != 4)
+        const items t(prog[n]);
+        if(t.size() != 4)
             fail(PyExc_ValueError, "an instruction is (op, type, operands, immediate)");
-        PyObject* op = PyDict_GetItemWithError(ops, item(t, 0));
+        PyObject* op = PyDict_GetItemWithError(ops, t[0]);
         if(op == nullptr)
             fail(PyExc_ValueError, "unknown element-wise operator");
-        PyObject* src   = item(t, 2);
-        d.insn[n].op    = static_cast<int>(integer(op));
-        d.insn[n].type  = static_cast<int>(integer(item(t, 1)));
-        d.insn[n].imm   = static_cast<float>(real(item(t, 3)));
-        const auto ns   = std::min<Py_ssize_t>(3, PySequence_Size(src));
+        const items src(t[2]);
+        d.insn[n].op   = static_cast<int>(integer(op));
+        d.insn[n].type = static_cast<int>(integer(t[1]));
+        d.insn[n].imm  = static_cast<float>(real(t[3]));
+        const auto ns  = std::min<Py_ssize_t>(3, src.size());
         for(Py_ssize_t j = 0; j < ns; ++j)
-            d.insn[n].src[j] = static_cast<int>(integer(item(src, j)));
+            d.insn[n].src[j] = static_cast<int>(integer(src[j]));
     }
     at::ScalarType t = at::kFloat;
     switch(d.insn[np - 1].type)
@@ -492,7 +501,7 @@ PyObject* pointwise(PyObject* const* a)
     case MGX_I32: t = at::kInt; break;
     default: fail(PyExc_KeyError, "result type of the last instruction");
     }
-    at::Tensor out = empty(sizes, t, tensor(item(ins, 0)));
+    at::Tensor out = empty(sizes, t, tensor(ins[0]));
     call("mgx_cuda_pointwise", [&] { return mgx_cuda_pointwise(&d, in, out.data_ptr(), stream()); });
     return wrap(std::move(out));
 }
