@@ -66,11 +66,9 @@ def test_static_scratch_matches_workspace_entry_point(cuda_device):
 
 
 def test_static_scratch_weight_streaming_route(cuda_device):
-    """[N,K] weights and at most 16 rows: the library's workspace for this shape is the
-    partial-sum area of the weight-streaming kernel, so the call runs that kernel with its tile
-    counters and partial sums inside the shared static array.  Two calls in a row (the second
-    one finds the first one's counters and sums there), each checked against the workspace
-    entry point and against the CPU oracle."""
+    """[N,K] weights and at most 16 rows: the announced workspace is within the limit (the weight-streaming
+    kernel needs none, its partial sums stay on the chip).  Calls in a row, each checked against the
+    workspace entry point and against the CPU oracle."""
     import torch
     from amdmigraphx_b200 import capi
     from oracle import mgx_oracle as O
@@ -87,7 +85,7 @@ def test_static_scratch_weight_streaming_route(cuda_device):
                            b_layout=capi.B_NK, scale_mode=capi.SCALE_PER_COL if fused else capi.SCALE_NONE,
                            act=capi.ACT_RELU if fused else capi.ACT_NONE, flags=0)
         need = lib.mgx_cuda_qgemm_workspace(ctypes.byref(d))
-        assert 0 < need <= lib.mgx_cuda_qgemm_static_scratch_limit()  # the streaming route is taken
+        assert 0 < need <= lib.mgx_cuda_qgemm_static_scratch_limit()
         odt = torch.float32 if fused else torch.int32
         ws = torch.empty(need, dtype=torch.uint8, device=cuda_device)
         want = capi.qgemm(a, b, b_layout=capi.B_NK, scale=scale if fused else None,
@@ -109,8 +107,8 @@ def test_static_scratch_weight_streaming_route(cuda_device):
 
 
 def test_static_scratch_falls_back_to_tiles_beyond_the_limit(cuda_device):
-    """[N,K] weights whose optional partial-sum area would not fit the static array: the call is
-    not rejected, it runs the tiled kernel, which needs no scratch."""
+    """[N,K] weights of more bytes than the static array holds, for which a kernel that kept partial sums of a
+    tile's columns in global memory would need more than it: the call is not rejected, whichever kernel serves it."""
     import torch
     from amdmigraphx_b200 import capi
     from oracle import mgx_oracle as O
@@ -121,8 +119,7 @@ def test_static_scratch_falls_back_to_tiles_beyond_the_limit(cuda_device):
     d = capi.QgemmDesc(M=M, N=N, K=K, batch=1, lda=K, ldb=K, ldd=N, stride_a=M * K, stride_b=N * K,
                        stride_d=M * N, ab_type=capi.I8, out_type=capi.I32, b_layout=capi.B_NK,
                        scale_mode=capi.SCALE_NONE, act=capi.ACT_NONE, flags=0)
-    if lib.mgx_cuda_qgemm_workspace(ctypes.byref(d)) <= lib.mgx_cuda_qgemm_static_scratch_limit():
-        pytest.skip("this shape's partial sums fit the static array")
+    assert N * K > lib.mgx_cuda_qgemm_static_scratch_limit()
     a = torch.from_numpy(rng.integers(-128, 128, size=(M, K), dtype=np.int8)).to(cuda_device)
     b = torch.from_numpy(rng.integers(-128, 128, size=(N, K), dtype=np.int8)).to(cuda_device)
     got = torch.zeros((M, N), dtype=torch.int32, device=cuda_device)
