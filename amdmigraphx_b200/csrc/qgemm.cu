@@ -1031,8 +1031,8 @@ extern "C" size_t mgx_cuda_qgemm_workspace(const mgx_qgemm_desc* d)
         return 0;
     if(d->b_layout != MGX_B_KN)
     {
-        // launches of at most 16 rows announce a minimal workspace, which callers of the interface lend
-        // and the kernel no longer needs: its partial sums stay on the chip
+        // [N,K] operands need no scratch.  Launches of at most 16 rows announced some when their kernel kept
+        // partial sums in global memory; the answer stays positive, nothing reads what is lent
         if(d->M > 0 and d->N > 0 and d->K > 0 and d->ab_type != MGX_F16 and qgemv_applicable(*d, false, false))
             return 256;
         return 0;
@@ -1211,16 +1211,10 @@ extern "C" int mgx_cuda_qgemm_static_scratch(const mgx_qgemm_desc* d, const void
         return MGX_E_INVALID_ARG;
     if(d->M <= 0 or d->N <= 0 or d->K <= 0 or d->batch <= 0)
         return MGX_E_INVALID_ARG;
-    size_t need = mgx_cuda_qgemm_workspace(d);
+    // only the re-laid-out copy of a [K,N] operand is kept in the scratch
+    const size_t need = d->b_layout == MGX_B_KN ? mgx_cuda_qgemm_workspace(d) : 0;
     if(need > static_scratch_bytes)
-    {
-        // a [K,N] operand has to be re-laid out into the scratch: no way around the limit.
-        // For [N,K] operands the scratch only enables the weight-streaming kernel for at most
-        // 16 rows; beyond the limit the tiled kernel runs, which needs none.
-        if(d->b_layout == MGX_B_KN)
-            return MGX_E_TOO_LARGE;
-        need = 0;
-    }
+        return MGX_E_TOO_LARGE;
     void* scratch = nullptr;
     if(need > 0)
     {

@@ -257,10 +257,10 @@ PyObject* qgemm(PyObject* const* a)
     d.ldd = md.ld, d.stride_d = md.stride;
     d.out_type = code_of(D.scalar_type());
     at::Tensor lent;
-    const size_t need = mgx_cuda_qgemm_workspace(&d);
-    if(need != 0 and workspace == nullptr)
+    if(b_layout == MGX_B_KN and workspace == nullptr)
     {
-        lent      = empty({static_cast<int64_t>(need)}, at::kByte, A);
+        // a [K,N] operand is re-laid out there; [N,K] operands take nothing
+        lent      = empty({static_cast<int64_t>(mgx_cuda_qgemm_workspace(&d))}, at::kByte, A);
         workspace = &lent;
     }
     const size_t have = workspace == nullptr ? 0 : static_cast<size_t>(workspace->numel());

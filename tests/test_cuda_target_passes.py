@@ -282,3 +282,9 @@ def test_llama_decoder_layer_lowers_to_int4_linears_cache_appends_and_decode_att
     # 13 launches: 4 linears, 2 RMSNorms, rotary, 2 cache appends, attention, residual add,
     # SwiGLU, residual add
     assert out.count("cuda::pointwise[") == 3
+
+
+def test_few_row_linear_gets_no_workspace():
+    out = _passes("c3_m16_n4096_k4096")
+    line = [l for l in out.splitlines() if "cuda::qgemm" in l][0]
+    assert "b_nk=1" in line and "has_workspace=0" in line

@@ -261,7 +261,7 @@ def test_skinny_quant_dot_fp8(cuda_device, M, N, K):
 
 
 def test_skinny_without_workspace_runs_as_tiles(cuda_device):
-    """The workspace is optional for [N,K] weights: without it the tiled kernel takes the call."""
+    """The workspace is optional for [N,K] weights: the call without it is accepted and right."""
     import ctypes
     import torch
     from amdmigraphx_b200 import capi
@@ -278,6 +278,21 @@ def test_skinny_without_workspace_runs_as_tiles(cuda_device):
     capi.check(lib.mgx_cuda_qgemm(ctypes.byref(desc), capi._ptr(at), capi._ptr(wt), capi._ptr(d), None,
                                   None, None, None, 0, capi._stream()), "mgx_cuda_qgemm")
     np.testing.assert_array_equal(d.cpu().numpy(), O.quant_dot_int8(a, w.T))
+
+
+@pytest.mark.parametrize("M", [1, 16, 17])
+def test_right_operand_in_nk_layout_takes_no_scratch(cuda_device, M):
+    """[N,K] weights are read in place: a call that is given its result and lent nothing allocates nothing."""
+    import torch
+    from amdmigraphx_b200 import capi
+    rng = np.random.default_rng(M)
+    a, w = _rand_i8(rng, (M, 512)), _rand_i8(rng, (384, 512))
+    at, wt = _t(a, cuda_device), _t(w, cuda_device)
+    out = torch.empty((M, 384), dtype=torch.int32, device=cuda_device)
+    before = torch.cuda.memory_stats()["allocation.all.allocated"]
+    capi.qgemm(at, wt, b_layout=capi.B_NK, out=out)
+    assert torch.cuda.memory_stats()["allocation.all.allocated"] == before
+    np.testing.assert_array_equal(out.cpu().numpy(), O.quant_dot_int8(a, w.T))
 
 
 @pytest.mark.parametrize("act", [None, "relu"])
