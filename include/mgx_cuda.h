@@ -391,6 +391,8 @@ typedef struct mgx_qgemm_desc
  * value is converted. */
 #define MGX_QGEMM_HALF_MATH 1
 
+/* Bytes of workspace: what a [K,N] right operand needs.  For [N,K] operands nothing is needed and nothing
+ * is read; with at most 16 rows of 8-bit A the answer is positive all the same, otherwise 0. */
 MGX_API size_t mgx_cuda_qgemm_workspace(const mgx_qgemm_desc* desc);
 MGX_API int mgx_cuda_qgemm(const mgx_qgemm_desc* desc,
                            const void* A,
@@ -424,8 +426,8 @@ typedef struct mgx_qgemm_qout
      * value whose fp16 bit pattern is h after dequantizelinear and bias: 65536 bytes in device memory
      * that the caller filled with activation + quantizelinear of every half (what a chain of fp16
      * operators makes of it, desc->act included).  The table is used where the launch takes the
-     * epilogue's vector path (M a multiple of 128, N of 16, aligned rows), otherwise the same values
-     * are computed.  Read only when the flag is set. */
+     * epilogue's vector path (any M, N a multiple of 16, aligned rows, no per-row scale), otherwise the
+     * same values are computed.  Read only when the flag is set. */
     const void* lut;
 } mgx_qgemm_qout;
 #define MGX_QOUT_LUT 1
@@ -448,20 +450,17 @@ MGX_API int mgx_cuda_qgemm_ex(const mgx_qgemm_desc* desc,
  * serving loop in which cudaMalloc's implicit device synchronisation is not acceptable, or
  * a host with a fixed memory budget.  It has no counterpart in the reference.
  * The scratch of the call - the re-laid-out copy of a [K,N] right operand (b_layout =
- * MGX_B_KN), or the tile counters and partial sums of the weight-streaming kernel that
- * [N,K] operands with at most 16 rows take - goes into a fixed
- * 16 MiB array that is part of this library's device image: every GPU that loads the
- * library holds those 16 MiB until the process exits.  Requests whose
- * mgx_cuda_qgemm_workspace() exceeds mgx_cuda_qgemm_static_scratch_limit() are rejected
- * with MGX_E_TOO_LARGE when the operand is [K,N]; with [N,K] operands (whose scratch is
- * optional) they run as tiles without scratch instead.  No cudaMalloc / cudaFree / allocating library routine is called.
+ * MGX_B_KN) - goes into a fixed 16 MiB array that is part of this library's device image:
+ * every GPU that loads the library holds those 16 MiB until the process exits.  A [K,N]
+ * operand whose mgx_cuda_qgemm_workspace() exceeds mgx_cuda_qgemm_static_scratch_limit() is
+ * rejected with MGX_E_TOO_LARGE; [N,K] operands need no scratch and have no limit.  No
+ * cudaMalloc / cudaFree / allocating library routine is called.
  * The first call on each device looks the array's device address up (one cheap runtime
  * query); make that first call before starting a stream capture on that device.
- * All calls on a device share the one array: two calls whose kernels may overlap on the
- * GPU (different streams without an ordering between them) race on it; calls on one stream
- * are safe.  The array keeps the previous call's bytes; what has to start at
- * zero (the tile counters of the weight-streaming kernel) is cleared by the call itself,
- * and every other byte the kernels read is rewritten by the same call first. */
+ * All calls on a device share the one array: two calls with [K,N] operands whose kernels may
+ * overlap on the GPU (different streams without an ordering between them) race on it; calls on
+ * one stream are safe.  The array keeps the previous call's bytes; every byte the kernels read
+ * is rewritten by the same call first. */
 MGX_API size_t mgx_cuda_qgemm_static_scratch_limit(void);
 MGX_API int mgx_cuda_qgemm_static_scratch(const mgx_qgemm_desc* desc,
                                           const void* A,
