@@ -191,10 +191,7 @@ template <int V, class IndexT>
 __global__ void __launch_bounds__(256) pointwise_kernel(const __grid_constant__ pw_args a)
 {
     const mgx_pw_desc& d = a.d;
-    // (packed int4 weights, which the int4 linears request before they wait, are 8-bit data)
-    if(d.insn[d.ninsns - 1].type == MGX_F16 or d.insn[d.ninsns - 1].type == MGX_F32)
-        grid_launch_dependents();
-    grid_dependency_wait();
+    grid_chain();
     float r[MGX_PW_MAXINSN][V];
     const int last       = d.ndim - 1;
     const IndexT nvec    = static_cast<IndexT>(a.total / V);

@@ -34,8 +34,9 @@
 // partial sums and counters in global memory and the planes are fetched again for every tile.  One row /
 // 16 rows, that form and this: 4096 x 4096 7.2 -> 6.4 us / 10.7 -> 8.2; 4096 x 11008 13.6 -> 9.8 /
 // 19.6 -> 17.0; 8192 x 1024 7.1 -> 4.4 / 8.8 -> 5.8; 7168 x 8192 11.8 -> 10.4 / 18.7 -> 17.1.
-// Launches are chained programmatically: the main kernel streams weights while the pre-kernel
-// (and the tail of the previous kernel of the stream) still runs.
+// Launches are chained programmatically: the main kernel streams weights while the pre-kernel still runs
+// - and not while what precedes that does, which may be what writes them (the pre-kernel lets it start only
+// after its own wait; with weights requested behind that kernel's back a decoder layer took 75.0 us, 76.5 so).
 // Only plain TMA loads; every wait is bounded.
 #include "common.cuh"
 #include "ptx.cuh"
@@ -220,8 +221,9 @@ __global__ void __launch_bounds__(TC_THREADS + (ESETS - 1) * 128, 1)
     {
         // ---------------------------------------------------- TMA producer
         // A stage = 4 groups of packed weights (two requests of 128 rows x 128 bytes).  The weights
-        // are constants of the model and are requested at once; the activation planes are written by
-        // the pre-kernel, whose completion is awaited before they are requested.
+        // are requested at once: whatever wrote them is complete, the pre-kernel having waited for it
+        // before it let this kernel start.  The activation planes are written by the pre-kernel, whose
+        // completion is awaited before they are requested.
         int tile = cluster, sg = sg_lo;
         const int head = min(nsuper, WST);
         int s = 0;

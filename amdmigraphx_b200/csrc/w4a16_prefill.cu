@@ -117,10 +117,13 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
     const int g_lo   = SPLIT ? G * rank / p.split : 0, g_hi = SPLIT ? G * (rank + 1) / p.split : G;
     const int rshift = 31 - __clz(p.group / PF_GROUP_K); // groups are powers of two
 
+    // everything the roles touch may be the previous kernel's: activations, packed weights, scales and zero
+    // points as its results, D as its input.  (The bounded waits below must not count its time either.)
+    grid_dependency_wait();
+
     if(warp == 0)
     {
         // ---------------------------------------------------- TMA producer
-        grid_dependency_wait(); // the activations are the previous kernel's output
         uint32_t s = 0, ph = 1;
         bool ok    = true;
         for(int t = first; ok and t < p.num_tiles; t += step)
@@ -158,7 +161,6 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
         const uint64_t bdesc0    = make_smem_desc_sw128(smem_u32(smem + PF_W_BYTES));
         uint32_t s = 0, ts = 0, tp = 0, lt = 0;
         bool ok    = true;
-        grid_dependency_wait(); // the bounded waits below must not count the previous kernel's time
         for(int t = first; ok and t < p.num_tiles; t += step, ++lt)
         {
             const uint32_t buf = lt & 1u;
@@ -287,7 +289,6 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
     else
     {
         // ---------------------------------------------------- epilogue
-        grid_dependency_wait(); // D may still be read by the previous kernel
         const int quarter = warp & 3;
         uint32_t lt       = 0;
         for(int t = first; t < p.num_tiles; t += step, ++lt)

@@ -10,6 +10,10 @@
  * cudaError_t reported by the CUDA runtime/driver.  Nothing throws across
  * this boundary.  There is no CPU fallback: an unsupported case is an error.
  *
+ * Calls on one stream take effect in order: every operand of a call - weights, scales and
+ * zero points included - may be the result of the call just before it.  (Kernels overlap with
+ * their predecessor's tail, but read nothing that it may still be writing.)
+ *
  * Device-side problems (a bounded wait inside a kernel ran out) are recorded
  * in a per-device status word, read with mgx_cuda_device_status().
  *
