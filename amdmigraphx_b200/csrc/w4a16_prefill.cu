@@ -3,20 +3,27 @@
 //   D[m,n] = sum_k a[m,k] * (q[n,k] - zp[n,k/group]) * s[n,k/group]
 //
 // as an fp16 x fp16 -> fp32 GEMM whose A operand is dequantised on the fly: the packed weights
-// of 128 output columns x 128 k arrive by TMA, four warps (one thread per weight row) turn them
+// of 128 output columns x 128 k arrive by TMA, eight warps (two threads per weight row) turn them
 // into fp16 values (q - zp) * s and write them straight into TENSOR MEMORY, and the MMAs read
 // their A operand from there; the B operand is the caller's fp16 activation matrix, fetched by
 // TMA as it lies in memory.  The dequantised weights never exist in shared or global memory
 // (the reference materialises them: src/onnx/parse_matmulnbits.cpp:85-158 IR on the ref target).
 //
-// CTA tile = 128 output columns x 128 activation rows, all of K; persistent over tiles.
-// CTA = 448 threads:
+// CTA tile = 128 output columns x 128 activation rows: all of K, persistent over tiles, or, where
+// tiles are few, a share of K and one tile.
+// The tensor core cuts its running sum at every step, which pulls a long one towards zero.  So a sum
+// runs over no more than half of K: the two halves of a tile have an accumulator each and are added in
+// the epilogue, and a third one lets the next tile begin meanwhile.  Mean relative error against 64-bit
+// sums, weights and activations of one sign, with one accumulator a tile and with two: K 4096 -2.3e-5 /
+// -1.1e-5, 11008 -5.8e-5 / -2.9e-5, 28672 -1.6e-4 / -8.1e-5.  Time of the same two, 512 rows: 12288 x 4096
+// 58.6 / 59.0 us, 4096 x 11008 57.0 / 53.3, 22016 x 4096 103.4 / 103.3; 1000 rows 12288 x 4096 119.1 / 117.1.
+// CTA = 576 threads:
 //   warp 0       TMA producer: per 128-k group 8 KB of packed weights and 2 x 16 KB of activations
 //   warps 2..5, 10..13  dequantise (nibbles -> fp16 pairs with byte permutes, one subtract and
 //                one multiply per pair) -> tcgen05.st
-//   warp 1       MMA issuer; two fp32 accumulators (128 columns of tensor memory each) take turns over
-//                the tiles
-//   warps 6..9   epilogue: tcgen05.ld, convert, store (consecutive lanes = consecutive n)
+//   warp 1       MMA issuer
+//   warps 6..9, 14..17  epilogue, half of a tile's activation rows each: tcgen05.ld, add, convert,
+//                store (consecutive lanes = consecutive n)
 // Only plain TMA loads; every wait is bounded.
 #include "common.cuh"
 #include "ptx.cuh"
@@ -31,11 +38,13 @@ constexpr int PF_STAGES  = 5;
 constexpr int PF_W_BYTES = PF_ROWS * PF_GROUP_K / 2;      // 8192
 constexpr int PF_A_ATOM  = PF_TOKENS * 128;               // 16384: 128 rows x 64 fp16
 constexpr int PF_STAGE   = PF_W_BYTES + 2 * PF_A_ATOM;    // 40960
-constexpr int PF_TSTAGES = 4;                             // A operand buffers in tensor memory
-constexpr int PF_A_COL0  = 256;
+constexpr int PF_TSTAGES = 2;                             // A operand buffers in tensor memory (four: no faster)
+constexpr int PF_ACCS    = 3;                             // accumulators there
+constexpr int PF_A_COL0  = PF_ACCS * PF_TOKENS;
 constexpr int PF_A_COLS  = PF_GROUP_K / 2;                // 64 columns per group
 constexpr int PF_SMEM    = PF_STAGES * PF_STAGE + 512 + 1024;
-constexpr int PF_THREADS = 448;
+constexpr int PF_THREADS = 576;
+constexpr int PF_EPI     = 256; // threads of the epilogue
 constexpr int PF_MAX_SPLIT = 8; // CTAs of a cluster
 
 struct pf_params
@@ -64,9 +73,9 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
     uint64_t* empty_bar     = full_bar + PF_STAGES;  // weights read (256) + MMAs retired (1)
     uint64_t* unp_bar       = empty_bar + PF_STAGES; // A operand in tensor memory
     uint64_t* tfree_bar     = unp_bar + PF_TSTAGES;  // MMAs that read it retired
-    uint64_t* accf_bar      = tfree_bar + PF_TSTAGES; // [2] accumulator ready
-    uint64_t* acce_bar      = accf_bar + 2;           // [2] accumulator drained
-    uint64_t* peer_bar      = acce_bar + 2;           // the cluster's partial results are in place
+    uint64_t* accf_bar      = tfree_bar + PF_TSTAGES; // accumulator ready
+    uint64_t* acce_bar      = accf_bar + PF_ACCS;     // accumulator drained
+    uint64_t* peer_bar      = acce_bar + PF_ACCS;          // the cluster's partial results are in place
     uint32_t* tmem_slot     = reinterpret_cast<uint32_t*>(peer_bar + 1);
     volatile uint32_t* abort_flag = tmem_slot + 1;
     float* part             = reinterpret_cast<float*>(smem); // [activation row][column], after the main loop
@@ -87,10 +96,10 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
             mbar_init(&unp_bar[s], 256);
             mbar_init(&tfree_bar[s], 1);
         }
-        for(int b = 0; b < 2; ++b)
+        for(int b = 0; b < PF_ACCS; ++b)
         {
             mbar_init(&accf_bar[b], 1);
-            mbar_init(&acce_bar[b], 4);
+            mbar_init(&acce_bar[b], PF_EPI / 32);
         }
         mbar_init(peer_bar, p.split);
         *abort_flag = 0;
@@ -115,6 +124,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
     const int first  = SPLIT ? static_cast<int>(blockIdx.x) / p.split : blockIdx.x;
     const int step   = SPLIT ? static_cast<int>(gridDim.x) / p.split : gridDim.x;
     const int g_lo   = SPLIT ? G * rank / p.split : 0, g_hi = SPLIT ? G * (rank + 1) / p.split : G;
+    // two segments of K, each with an accumulator (a CTA's share of K that is one of several: one)
+    const int g_mid  = SPLIT or G == 1 ? g_hi : (g_lo + g_hi) / 2;
     const int rshift = 31 - __clz(p.group / PF_GROUP_K); // groups are powers of two
 
     // everything the roles touch may be the previous kernel's: activations, packed weights, scales and zero
@@ -154,51 +165,50 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
     {
         // ---------------------------------------------------- MMA issuer
         // D f32 += A f16 (weights, tensor memory) * B f16 (activation rows, K-major shared
-        // memory); M = 128, N = 128, K = 16 per instruction.  Two accumulators take turns, so that the
-        // epilogue of a tile overlaps the main loop of the next.  (As one accumulator per half of a
-        // group's k, added in the epilogue, every tile waited for the one before to be stored.)
+        // memory); M = 128, N = 128, K = 16 per instruction.  Three accumulators take turns over the
+        // segments, so that the epilogue of a tile overlaps the main loop of the next.
         constexpr uint32_t idesc = make_idesc(1u, 0u, 0u, PF_ROWS, PF_TOKENS);
         const uint64_t bdesc0    = make_smem_desc_sw128(smem_u32(smem + PF_W_BYTES));
-        uint32_t s = 0, ts = 0, tp = 0, lt = 0;
+        uint32_t s = 0, ts = 0, tp = 0, buf = 0, bp = 1;
         bool ok    = true;
-        for(int t = first; ok and t < p.num_tiles; t += step, ++lt)
-        {
-            const uint32_t buf = lt & 1u;
-            if(not mbar_wait_warp(&acce_bar[buf], ((lt >> 1) & 1u) ^ 1u, abort_flag, 4))
-                break;
-            tc_fence_after_sync();
-            const uint32_t d_tmem = tmem_base + buf * PF_TOKENS;
-            for(int g = g_lo; g < g_hi; ++g)
+        for(int t = first; ok and t < p.num_tiles; t += step)
+            for(int g = g_lo; ok and g < g_hi;)
             {
-                // implies that the stage's TMA requests have landed
-                if(not mbar_wait_warp(&unp_bar[ts], tp, abort_flag, 5))
-                {
-                    ok = false;
-                    break;
-                }
+                const int g0 = g, g1 = g0 < g_mid ? g_mid : g_hi;
+                ok = mbar_wait_warp(&acce_bar[buf], bp, abort_flag, 4);
                 tc_fence_after_sync();
-                if(elect_one())
+                const uint32_t d_tmem = tmem_base + buf * PF_TOKENS;
+                for(; ok and g < g1; ++g)
                 {
-                    const uint64_t bdesc  = bdesc0 + static_cast<uint64_t>((s * PF_STAGE) >> 4);
-                    const uint32_t a_tmem = tmem_base + PF_A_COL0 + ts * PF_A_COLS;
+                    // implies that the stage's TMA requests have landed
+                    ok = mbar_wait_warp(&unp_bar[ts], tp, abort_flag, 5);
+                    if(not ok)
+                        break;
+                    tc_fence_after_sync();
+                    if(elect_one())
+                    {
+                        const uint64_t bdesc  = bdesc0 + static_cast<uint64_t>((s * PF_STAGE) >> 4);
+                        const uint32_t a_tmem = tmem_base + PF_A_COL0 + ts * PF_A_COLS;
 #pragma unroll
-                    for(int k = 0; k < 8; ++k) // (64 k per 128-byte atom)
-                        mma_f16_tmem_a(d_tmem, a_tmem + k * 8,
-                                       bdesc + static_cast<uint64_t>(((k >> 2) * PF_A_ATOM + (k & 3) * 32) >> 4), idesc,
-                                       (g != g_lo or k != 0) ? 1u : 0u);
-                    tc_commit(&tfree_bar[ts]);
-                    tc_commit(&empty_bar[s]);
-                    if(g == g_hi - 1)
-                        tc_commit(&accf_bar[buf]);
+                        for(int k = 0; k < 8; ++k) // (64 k per 128-byte atom)
+                            mma_f16_tmem_a(d_tmem, a_tmem + k * 8,
+                                           bdesc + static_cast<uint64_t>(((k >> 2) * PF_A_ATOM + (k & 3) * 32) >> 4), idesc,
+                                           (g != g0 or k != 0) ? 1u : 0u);
+                        tc_commit(&tfree_bar[ts]);
+                        tc_commit(&empty_bar[s]);
+                        if(g == g1 - 1)
+                            tc_commit(&accf_bar[buf]);
+                    }
+                    if(++s == PF_STAGES)
+                        s = 0;
+                    if(++ts == PF_TSTAGES)
+                        ts = 0, tp ^= 1u;
                 }
-                if(++s == PF_STAGES)
-                    s = 0;
-                if(++ts == PF_TSTAGES)
-                    ts = 0, tp ^= 1u;
+                if(++buf == PF_ACCS)
+                    buf = 0, bp ^= 1u;
             }
-        }
     }
-    else if(warp < 6 or warp >= 10)
+    else if(warp < 6 or (warp >= 10 and warp < 14))
     {
         // ---------------------------------------------------- dequantise: nibbles -> fp16
         // Two threads per weight row (warps 2..5 take the first 64 k of a group, warps 10..13 the
@@ -290,35 +300,55 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
     {
         // ---------------------------------------------------- epilogue
         const int quarter = warp & 3;
-        uint32_t lt       = 0;
-        for(int t = first; t < p.num_tiles; t += step, ++lt)
+        const int c0      = warp >= 14 ? PF_TOKENS / 2 : 0; // this warp's activation rows of the tile
+        const int segs    = g_mid < g_hi ? 2 : 1;
+        uint32_t buf = 0, bp = 0;
+        for(int t = first; t < p.num_tiles; t += step)
         {
             const int64_t n  = static_cast<int64_t>(t / p.tiles_m) * PF_ROWS + quarter * 32 + lane;
             const int64_t m0 = static_cast<int64_t>(t % p.tiles_m) * PF_TOKENS;
-            const uint32_t buf = lt & 1u;
-            if(not mbar_wait_warp(&accf_bar[buf], (lt >> 1) & 1u, abort_flag, 3))
+            const uint32_t buf0 = buf;
+            bool ok = true;
+            for(int i = 0; ok and i < segs; ++i)
+            {
+                ok = mbar_wait_warp(&accf_bar[buf], bp, abort_flag, 3);
+                if(++buf == PF_ACCS)
+                    buf = 0, bp ^= 1u;
+            }
+            if(not ok)
                 break;
+            const uint32_t buf1 = buf0 + 1 == PF_ACCS ? 0 : buf0 + 1;
             tc_fence_after_sync();
-            const uint32_t tbase = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * PF_TOKENS;
+            const uint32_t tbase = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + c0;
 #pragma unroll 1
             for(int c = 0; c < PF_TOKENS / 32; ++c)
             {
-                uint32_t acc[32];
-                tmem_ld_32x32b_x32(tbase + c * 32, acc);
-                tmem_ld_wait();
+                uint32_t acc[16];
+                tmem_ld_32x32b_x16(tbase + buf0 * PF_TOKENS + c * 16, acc);
+                if(not SPLIT and segs == 2)
+                {
+                    uint32_t acc1[16];
+                    tmem_ld_32x32b_x16(tbase + buf1 * PF_TOKENS + c * 16, acc1);
+                    tmem_ld_wait();
+#pragma unroll
+                    for(int j = 0; j < 16; ++j)
+                        acc[j] = __float_as_uint(__uint_as_float(acc[j]) + __uint_as_float(acc1[j]));
+                }
+                else
+                    tmem_ld_wait();
                 if constexpr(SPLIT)
                 {
                     // (every request has landed and every MMA has read: the ring is free)
 #pragma unroll
-                    for(int j = 0; j < 32; ++j)
-                        part[(c * 32 + j) * PF_ROWS + quarter * 32 + lane] = __uint_as_float(acc[j]);
+                    for(int j = 0; j < 16; ++j)
+                        part[(c0 + c * 16 + j) * PF_ROWS + quarter * 32 + lane] = __uint_as_float(acc[j]);
                 }
                 else if(n < p.N)
                 {
 #pragma unroll
-                    for(int j = 0; j < 32; ++j)
+                    for(int j = 0; j < 16; ++j)
                     {
-                        const int64_t m = m0 + c * 32 + j;
+                        const int64_t m = m0 + c0 + c * 16 + j;
                         if(m < p.M)
                             p.D[m * p.ldd + n] = __float2half_rn(__uint_as_float(acc[j]));
                     }
@@ -327,12 +357,16 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
             tc_fence_before_sync();
             __syncwarp();
             if(lane == 0)
-                mbar_arrive(&acce_bar[buf]);
+            {
+                mbar_arrive(&acce_bar[buf0]);
+                if(segs == 2)
+                    mbar_arrive(&acce_bar[buf1]);
+            }
             if constexpr(SPLIT)
             {
                 // CTA r adds up the r-th share of the tile's columns, four at a time
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                const int et = threadIdx.x - 192;
+                asm volatile("bar.sync 1, %0;" ::"n"(PF_EPI) : "memory");
+                const int et = static_cast<int>(threadIdx.x) - (warp >= 14 ? 320 : 192);
                 if(et < p.split)
                     cluster_arrive(peer_bar, et);
                 if(__all_sync(0xffffffffu, mbar_wait_cluster_bounded(peer_bar, 0u, abort_flag, 6)))
@@ -340,8 +374,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
                     const int share = PF_ROWS / p.split, per = share / 4;
                     const int col   = rank * share + et % per * 4;
                     const int64_t n4 = static_cast<int64_t>(t / p.tiles_m) * PF_ROWS + col;
-#pragma unroll 2
-                    for(int m = et / per; m < PF_TOKENS and m0 + m < p.M; m += 128 / per)
+                    for(int m = et / per; m < PF_TOKENS and m0 + m < p.M; m += PF_EPI / per)
                     {
                         float v[PF_MAX_SPLIT][4], sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
