@@ -315,7 +315,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
                 if(++buf == PF_ACCS)
                     buf = 0, bp ^= 1u;
             }
-            if(not ok)
+            // (in a cluster a wait that gave up goes on without waiting: the barriers below need every thread)
+            if(not SPLIT and not ok)
                 break;
             const uint32_t buf1 = buf0 + 1 == PF_ACCS ? 0 : buf0 + 1;
             tc_fence_after_sync();
@@ -369,7 +370,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
                 const int et = static_cast<int>(threadIdx.x) - (warp >= 14 ? 320 : 192);
                 if(et < p.split)
                     cluster_arrive(peer_bar, et);
-                if(__all_sync(0xffffffffu, mbar_wait_cluster_bounded(peer_bar, 0u, abort_flag, 6)))
+                if(ok and __all_sync(0xffffffffu, mbar_wait_cluster_bounded(peer_bar, 0u, abort_flag, 6)))
                 {
                     const int share = PF_ROWS / p.split, per = share / 4;
                     const int col   = rank * share + et % per * 4;
