@@ -27,7 +27,9 @@
 // Only plain TMA loads; every wait is bounded.
 #include "common.cuh"
 #include "ptx.cuh"
+#include <algorithm>
 #include <cuda_fp16.h>
+#include <mutex>
 
 namespace mgx {
 
@@ -438,6 +440,49 @@ int encode_rows(CUtensorMap* map, CUtensorMapDataType type, const void* base, ui
     return r == CUDA_SUCCESS ? MGX_OK : MGX_E_INVALID_ARG;
 }
 
+void configure(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2], int clusters, int split, cudaStream_t stream)
+{
+    cfg                  = cudaLaunchConfig_t{};
+    cfg.gridDim          = dim3(static_cast<unsigned>(clusters * split));
+    cfg.blockDim         = dim3(PF_THREADS);
+    cfg.dynamicSmemBytes = PF_SMEM;
+    cfg.stream           = stream;
+    attr[0].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id               = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = static_cast<unsigned>(split);
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs    = attr;
+    cfg.numAttrs = split > 1 ? 2 : 1;
+}
+
+// Clusters of `split` CTAs that fit the device at once (asked once per device): a cluster lies inside a
+// GPC, so that fewer fit than the SMs alone would allow.
+int max_clusters(int split)
+{
+    static std::mutex m;
+    static int cached[64][PF_MAX_SPLIT + 1] = {};
+    int dev = 0;
+    if(cudaGetDevice(&dev) != cudaSuccess or dev < 0 or dev >= 64)
+        return device_sm_count() / (2 * split);
+    std::lock_guard<std::mutex> lock(m);
+    int& n = cached[dev][split];
+    if(n == 0)
+    {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute attr[2];
+        configure(cfg, attr, device_sm_count() / split, split, nullptr);
+        attr[0]      = attr[1];
+        cfg.numAttrs = 1;
+        if(cudaOccupancyMaxActiveClusters(&n, w4a16_prefill_kernel<true>, &cfg) != cudaSuccess or n < 1)
+        {
+            (void)cudaGetLastError();
+            n = device_sm_count() / (2 * split);
+        }
+    }
+    return n;
+}
+
 } // namespace
 
 bool w4a16_prefill_applicable(const mgx_w4_desc& d, const void* A, const void* Bp)
@@ -477,31 +522,23 @@ int w4a16_prefill_launch(const mgx_w4_desc& d, const void* A, const void* Bp, co
     p.zp_const       = d.zp_const;
     p.tiles_m        = static_cast<int>(ceil_div(d.M, PF_TOKENS));
     p.num_tiles      = static_cast<int>(ceil_div(d.N, PF_ROWS)) * p.tiles_m;
-    const int sms  = device_sm_count();
     // Few tiles leave SMs idle: a cluster shares a tile's K, each CTA at least four groups, and adds its
     // partial results through distributed shared memory (24 tokens, 4096 x 11008, 32 tiles: 44 us in one
-    // CTA each, 18 us).
+    // CTA each, 17 us).  Only where all the clusters run at once, as one left over costs a second wave: 16 tiles
+    // of K 4096, eight CTAs each 17.6 us, four 10.7; 36 tiles of K 11008, four 36.3, two 29.3.
+    rc = ensure_smem_optin(reinterpret_cast<const void*>(w4a16_prefill_kernel<true>), PF_SMEM);
+    if(rc != MGX_OK)
+        return rc;
     p.split = 1;
-    while(p.split < PF_MAX_SPLIT and p.num_tiles * p.split * 2 <= sms and d.K / PF_GROUP_K >= 8 * p.split)
-        p.split *= 2;
-    const int grid = p.split > 1 ? p.num_tiles * p.split : (p.num_tiles < sms ? p.num_tiles : sms);
+    for(int s = 2; s <= PF_MAX_SPLIT and d.K / PF_GROUP_K >= 4 * s and p.num_tiles <= max_clusters(s); s *= 2)
+        p.split = s;
     auto* kernel = p.split > 1 ? w4a16_prefill_kernel<true> : w4a16_prefill_kernel<false>;
     rc           = ensure_smem_optin(reinterpret_cast<const void*>(kernel), PF_SMEM);
     if(rc != MGX_OK)
         return rc;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim          = dim3(static_cast<unsigned>(grid));
-    cfg.blockDim         = dim3(PF_THREADS);
-    cfg.dynamicSmemBytes = PF_SMEM;
-    cfg.stream           = stream;
+    cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
-    attr[0].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id               = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = static_cast<unsigned>(p.split);
-    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-    cfg.attrs    = attr;
-    cfg.numAttrs = p.split > 1 ? 2 : 1;
+    configure(cfg, attr, p.split > 1 ? p.num_tiles : std::min(p.num_tiles, device_sm_count()), p.split, stream);
     return static_cast<int>(cudaLaunchKernelEx(&cfg, kernel, tw, ta, p));
 }
 
