@@ -38,28 +38,12 @@
 // - and not while what precedes that does, which may be what writes them (the pre-kernel lets it start only
 // after its own wait; with weights requested behind that kernel's back a decoder layer took 75.0 us, 76.5 so).
 // Only plain TMA loads; every wait is bounded.
-#include "common.cuh"
-#include "ptx.cuh"
-#include "w4a16_acts.cuh"
+#include "w4a16_decode.cuh"
 #include <algorithm>
-#include <cuda_fp16.h>
 #include <mutex>
 
 namespace mgx {
-namespace { // (names shared with w4a16_tc.cu)
-
-constexpr int TC_ROWS     = 128; // output columns (weight rows) per CTA tile = UMMA M
-constexpr int TC_GROUP_K  = 128; // k per group
-constexpr int TC_SUPER    = 4;   // groups per work item (each row gives 256 contiguous bytes)
-constexpr int TC_PACKED   = TC_ROWS * TC_GROUP_K / 2; // 8192 bytes of packed weights per group
-constexpr int TC_WSTAGE   = TC_SUPER * TC_PACKED;     // 32768
-constexpr int TC_TSTAGES  = 2;   // A operand buffers in tensor memory
-constexpr int TC_THREADS  = 480;
-constexpr int TC_ISSUERS  = 4;   // MMA-issuing threads, one per group of a work item
-constexpr int TC_ACC_COLS = 128; // accumulator columns per buffer (two buffers)
-constexpr int TC_A_COL0   = 256; // first tensor-memory column of the A operand buffers
-constexpr int TC_A_COLS   = TC_GROUP_K / 4; // 32 columns per group
-constexpr int TC_EPI      = 3 * 128 * (5 + 3 + 2) * 4 + 64; // epilogue metadata
+namespace { // (names that w4a16_tc.cu has too)
 
 constexpr int TC_MAX_SPLIT  = 8; // CTAs of a cluster; divides TC_ROWS
 constexpr int TC_MAX_STAGES = 5;
@@ -73,16 +57,8 @@ constexpr size_t tc_fixed(int items, int rows)
     return static_cast<size_t>(items) * TC_SUPER * NB * TC_GROUP_K + 512 + TC_EPI + TC_XBUFS * rows * TC_ROWS * 4 + 1024;
 }
 
-struct tc_params
+struct tc_params : tc_operands
 {
-    const __half* scales;
-    const uint8_t* zp; // may be null
-    const float* sa;   // [K/128][MB] activation scale of every (group, row)
-    const int* sv;     // [K/128][MB] per-group sums of the quantised activations
-    __half* D;
-    int64_t N, K, ldd;
-    int M;
-    int group, groups_per_row, zp_const;
     int tiles, clusters, split; // tiles of 128 columns; clusters; CTAs of a cluster
     int items, stages;          // most work items of a share of K; stages of the ring
 };
@@ -117,24 +93,12 @@ struct tc_walk
     }
 };
 
-// MR: activation rows folded by the epilogue (M <= MR <= MB).
-// RAW: the weight operand of a group is [64 bytes of low nibbles | the 64 packed bytes] and every
-// activation row has 4 rows in the B operand (see the pre-kernel); otherwise it is the 128
-// nibbles unpacked to bytes and 2 rows.  RAW costs one logic operation per eight weights
-// instead of three, and twice the accumulator columns per activation row.
-// ESETS: sets of four epilogue warps; with two, each set folds half of the MR rows (the second
-// set is warps 15..18).
-template <int NB, int MR, bool RAW, int ESETS>
-__global__ void __launch_bounds__(TC_THREADS + (ESETS - 1) * 128, 1)
-    w4a16_cluster_kernel(const __grid_constant__ CUtensorMap tmap_w,
-                    const __grid_constant__ CUtensorMap tmap_a,
-                    const tc_params p)
+template <class FORM>
+__global__ void __launch_bounds__(FORM::THREADS, 1)
+    w4a16_cluster_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a, const tc_params p)
 {
-    constexpr int CPM    = RAW ? 4 : 2;      // accumulator columns per activation row
-    constexpr int MB     = NB / CPM;         // padded activation rows
-    constexpr int GPP    = TC_ACC_COLS / NB; // groups per pass (one accumulator buffer): 8 or 4
-    constexpr int XROWS  = MB;               // rows of a partial result
-    constexpr int ABYTES = NB * TC_GROUP_K;  // activation rows of one group
+    constexpr int NB = FORM::NB, CPM = FORM::CPM, GPP = FORM::GPP, ABYTES = FORM::ABYTES, MRW = FORM::MRW, ESETS = FORM::ESETS;
+    constexpr int XROWS = FORM::MB; // rows of a partial result
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw_addr = smem_u32(smem_raw);
     uint8_t* smem           = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
@@ -153,13 +117,7 @@ __global__ void __launch_bounds__(TC_THREADS + (ESETS - 1) * 128, 1)
     uint64_t* peer_bar      = acts_bar + 1;     // the whole cluster's partial results are in place
     uint32_t* tmem_slot     = reinterpret_cast<uint32_t*>(peer_bar + 1);
     volatile uint32_t* abort_flag = tmem_slot + 1;
-    // epilogue metadata, three buffers each: per output column the aligned 32-bit words that
-    // hold the scales (at most 5) and zero points (at most 3) of a pass, GPP x MB activation
-    // group sums and group scales
-    uint32_t* epi_sw = reinterpret_cast<uint32_t*>(bar_base + 512);     // [3][128][5]
-    uint32_t* epi_zw = epi_sw + 3 * 128 * 5;                            // [3][128][3]
-    int* epi_sv      = reinterpret_cast<int*>(epi_zw + 3 * 128 * 3);    // [3][128]
-    float* epi_sa    = reinterpret_cast<float*>(epi_sv + 3 * 128);      // [3][128]
+    const tc_meta meta(bar_base + 512);
     float* part      = reinterpret_cast<float*>(bar_base + 512 + TC_EPI); // [TC_XBUFS][XROWS][128]
 
     const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
@@ -317,21 +275,8 @@ __global__ void __launch_bounds__(TC_THREADS + (ESETS - 1) * 128, 1)
     else if(warp == 13 or warp == 14)
     {
         // ---------------------------------------------------- epilogue metadata, up to 3 passes ahead
-        // cp.async copies of the aligned words around the scales and zero points of a pass
-        // (consecutive lanes copy consecutive words of a column's run, so a request touches
-        // few sectors) and of the activation group sums.  Each of the two warps serves 64
-        // output columns.
+        // Each of the two warps serves 64 output columns.
         grid_dependency_wait(); // sv and sa come from the pre-kernel
-        const int half  = warp - 13;
-        const int rshift = 31 - __clz(p.group / TC_GROUP_K); // groups are powers of two
-        const uint32_t sbase0 = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(p.scales) & 3u);
-        const uint32_t zbase0 = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(p.zp) & 3u);
-        const char* sptr = reinterpret_cast<const char*>(p.scales) - sbase0; // 4-byte aligned
-        const char* zptr = reinterpret_cast<const char*>(p.zp) - zbase0;
-        auto cp_async4 = [](const void* dst, const void* src) {
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src)
-                         : "memory");
-        };
         tc_walk walk = walk0;
         int tile, g0, count;
         bool seg_last;
@@ -340,60 +285,17 @@ __global__ void __launch_bounds__(TC_THREADS + (ESETS - 1) * 128, 1)
             const uint32_t vb = pc % 3u;
             if(not mbar_wait_bounded(&mfree_bar[vb], ((pc / 3u) & 1u) ^ 1u, abort_flag, 9))
                 break;
-            const int gi0 = g0 >> rshift;
-            const int ng  = ((g0 + count - 1) >> rshift) - gi0 + 1;
-            const int n0  = tile * TC_ROWS + half * 64;
-            // scales: up to 5 words per column
-#pragma unroll 2
-            for(int idx = lane; idx < 64 * 5; idx += 32)
-            {
-                const int r = idx / 5, w = idx - r * 5;
-                const int n = min(n0 + r, static_cast<int>(p.N) - 1);
-                // byte offsets from the aligned base: first scale, end of the run
-                const uint32_t s = sbase0 + static_cast<uint32_t>(n * p.groups_per_row + gi0) * 2u;
-                const uint32_t a = s & ~3u;
-                const int nw     = static_cast<int>((((s + ng * 2 + 3u) & ~3u) - a) >> 2);
-                if(w < nw)
-                    cp_async4(epi_sw + (vb * 128 + half * 64 + r) * 5 + w, sptr + a + 4 * w);
-            }
-            if(p.zp != nullptr)
-            {
-#pragma unroll 2
-                for(int idx = lane; idx < 64 * 3; idx += 32)
-                {
-                    const int r = idx / 3, w = idx - r * 3;
-                    const int n = min(n0 + r, static_cast<int>(p.N) - 1);
-                    const uint32_t z = zbase0 + static_cast<uint32_t>(n * p.groups_per_row + gi0);
-                    const uint32_t a = z & ~3u;
-                    const int nw     = static_cast<int>((((z + ng + 3u) & ~3u) - a) >> 2);
-                    if(w < nw)
-                        cp_async4(epi_zw + (vb * 128 + half * 64 + r) * 3 + w, zptr + a + 4 * w);
-                }
-            }
-            // group sums and group scales: count x MB words each, half of them per warp
-            for(int i = half * 64 + lane; i < count * MB; i += 32)
-                if(i < half * 64 + 64)
-                {
-                    cp_async4(epi_sv + vb * 128 + i, p.sv + static_cast<int64_t>(g0) * MB + i);
-                    cp_async4(epi_sa + vb * 128 + i, p.sa + static_cast<int64_t>(g0) * MB + i);
-                }
-            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(
-                             smem_u32(&meta_bar[vb]))
-                         : "memory");
+            tc_stage_metadata<FORM::MB>(p, meta, vb, warp - 13, lane, tile, g0, count);
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&meta_bar[vb])) : "memory");
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
     }
     else if(warp < 6)
     {
         // ---------------------------------------------------- unpack: nibbles -> bytes
-        // One thread per weight row: 64 packed bytes per group from shared memory (128-byte
-        // swizzle, so a quarter warp's 16-byte reads fall in eight different bank groups), 32
-        // words to this row's lane of tensor memory: either the nibbles as bytes (inside every
-        // 8 k the evens first, then the odds; the activation rows are stored in the same order)
-        // or the low nibbles followed by the packed bytes as they are (RAW).
+        // one thread per weight row
         const int row            = (warp & 3) * 32 + lane;
         const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
-        const int sw             = row & 7;
         int sg                   = sg_lo;
         int s                    = 0;
         uint32_t ph              = 0;
@@ -408,39 +310,7 @@ __global__ void __launch_bounds__(TC_THREADS + (ESETS - 1) * 128, 1)
                 break;
             tc_fence_after_sync();
             const int cnt = min(TC_SUPER, G - sg * TC_SUPER);
-#pragma unroll
-            for(int q = 0; q < TC_SUPER; ++q)
-            {
-                if(q < cnt)
-                {
-                    // [pair of groups][row][128 bytes], 16-byte chunks swizzled by the row
-                    const uint8_t* pk = smem + s * TC_WSTAGE + (q >> 1) * (2 * TC_PACKED) + row * 128;
-                    uint32_t u[32];
-#pragma unroll
-                    for(int c = 0; c < 4; ++c)
-                    {
-                        const uint4 w =
-                            *reinterpret_cast<const uint4*>(pk + ((((q & 1) * 4 + c) ^ sw) << 4));
-                        if constexpr(RAW)
-                        {
-                            u[4 * c + 0] = w.x & 0x0F0F0F0Fu, u[16 + 4 * c + 0] = w.x;
-                            u[4 * c + 1] = w.y & 0x0F0F0F0Fu, u[16 + 4 * c + 1] = w.y;
-                            u[4 * c + 2] = w.z & 0x0F0F0F0Fu, u[16 + 4 * c + 2] = w.z;
-                            u[4 * c + 3] = w.w & 0x0F0F0F0Fu, u[16 + 4 * c + 3] = w.w;
-                        }
-                        else
-                        {
-                            u[8 * c + 0] = w.x & 0x0F0F0F0Fu, u[8 * c + 1] = (w.x >> 4) & 0x0F0F0F0Fu;
-                            u[8 * c + 2] = w.y & 0x0F0F0F0Fu, u[8 * c + 3] = (w.y >> 4) & 0x0F0F0F0Fu;
-                            u[8 * c + 4] = w.z & 0x0F0F0F0Fu, u[8 * c + 5] = (w.z >> 4) & 0x0F0F0F0Fu;
-                            u[8 * c + 6] = w.w & 0x0F0F0F0Fu, u[8 * c + 7] = (w.w >> 4) & 0x0F0F0F0Fu;
-                        }
-                    }
-                    tmem_st_32x32b_x32(tmem_base + lane_addr + TC_A_COL0 +
-                                           (t * TC_SUPER + q) * TC_A_COLS,
-                                       u);
-                }
-            }
+            tc_unpack_item<FORM::RAW>(smem + s * TC_WSTAGE, row, cnt, tmem_base + lane_addr + TC_A_COL0 + t * TC_SUPER * TC_A_COLS);
             mbar_arrive(&empty_bar[s]); // the packed blocks are in registers
             tmem_st_wait();
             tc_fence_before_sync();
@@ -454,63 +324,16 @@ __global__ void __launch_bounds__(TC_THREADS + (ESETS - 1) * 128, 1)
     else
     {
         // ---------------------------------------------------- epilogue: fold the groups
-        // Scale, zero point and activation group sums of a pass are already in shared memory
-        // (metadata warps).  Column 2 m of a group's accumulator is P_hi, column 2 m + 1 P_lo
-        // of activation row m; only the MR rows in use are read.  All arithmetic stays off
-        // the conversion pipe except one half -> float per group: |P_hi|, |P_lo| < 2^18.
         grid_dependency_wait(); // sa comes from the pre-kernel, D may still be read by an earlier one
-        constexpr int MRW = MR / ESETS;          // rows this warp folds ...
         const int eset    = warp >= 15 ? 1 : 0;
-        const int m0      = eset * MRW;          // ... starting at this one
+        const int m0      = eset * MRW;          // first of the rows this warp folds
         const int quarter = warp & 3;
         const int col     = quarter * 32 + lane; // output column inside the tile = TMEM lane
-        const int rshift  = 31 - __clz(p.group / TC_GROUP_K); // groups are powers of two
-        const uint32_t sbase0 = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(p.scales) & 3u);
-        const uint32_t zbase0 = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(p.zp) & 3u);
         float out[MRW];
 #pragma unroll
         for(int m = 0; m < MRW; ++m)
             out[m] = 0.0f;
         tc_walk walk = walk0;
-        // one group: out[m] += sc sa[m] (Q[m] - z Sv[m]) with Q = sum_k q a_int, in exact integer
-        // arithmetic up to the one conversion.  soff / zoff: byte offset of the group's scale /
-        // zero point inside this column's staged words
-        constexpr int C  = CPM * MRW; // accumulator columns read per group
-        const bool has_zp = p.zp != nullptr;
-        auto fold = [&](const uint32_t(&acc)[C], int gl, uint32_t vb, uint32_t soff, uint32_t zoff) {
-            const uint32_t sw = epi_sw[(vb * 128 + col) * 5 + (soff >> 2)];
-            const uint32_t sh = (soff & 2u) ? sw >> 16 : sw & 0xFFFFu;
-            float sc          = __half2float(__ushort_as_half(static_cast<unsigned short>(sh)));
-            // without zero points the staged word is not meaningful and not used
-            const uint32_t zw = epi_zw[(vb * 128 + col) * 3 + (has_zp ? zoff >> 2 : 0u)];
-            int z = has_zp ? static_cast<int>((zw >> (8u * (zoff & 3u))) & 0xFFu) : p.zp_const;
-            if constexpr(RAW)
-            {
-                sc *= 0.0625f; // Q is computed times 16
-                z *= 16;
-            }
-            const int* svb   = epi_sv + vb * 128 + gl * MB + m0;
-            const float* sab = epi_sa + vb * 128 + gl * MB + m0;
-#pragma unroll
-            for(int m = 0; m < MRW; ++m)
-            {
-                int q;
-                if constexpr(RAW)
-                {
-                    // columns: sum L e_h, 16 sum q_odd o_h, sum L e_l, 16 sum q_odd o_l;
-                    // 16 Q = 2048 E_h + 128 O_h + 16 E_l + O_l
-                    q = static_cast<int>(acc[4 * m]) * 2048 + static_cast<int>(acc[4 * m + 3]);
-                    q = static_cast<int>(acc[4 * m + 1]) * 128 + q;
-                    q = static_cast<int>(acc[4 * m + 2]) * 16 + q;
-                }
-                else
-                    q = static_cast<int>(acc[2 * m]) * 128 + static_cast<int>(acc[2 * m + 1]);
-                q      = q - z * svb[m];
-                out[m] = fmaf(sc * sab[m], static_cast<float>(q), out[m]);
-            }
-        };
-        // groups read from tensor memory per trip (all loads in flight before the first fold)
-        constexpr int TR = C <= 4 ? 8 : (C <= 8 ? 4 : 2);
         constexpr int ETHREADS = 128 * ESETS;
         const int et           = (eset == 1 ? warp - 15 : warp - 6) * 32 + lane + eset * 128;
         bool dead              = false; // a wait gave up: go on without waiting, the barriers need every thread
@@ -546,43 +369,8 @@ __global__ void __launch_bounds__(TC_THREADS + (ESETS - 1) * 128, 1)
                              not mbar_wait_warp(&accf_bar[buf], (pc >> 1) & 1u, abort_flag, 3)))
                 dead = true;
             tc_fence_after_sync();
-            const int gi0 = g0 >> rshift;
-            const int n   = min(tile * TC_ROWS + col, static_cast<int>(p.N) - 1);
-            const uint32_t sbyte =
-                (sbase0 + static_cast<uint32_t>(n * p.groups_per_row + gi0) * 2u) & 3u;
-            const uint32_t zbyte = (zbase0 + static_cast<uint32_t>(n * p.groups_per_row + gi0)) & 3u;
-            // quantisation group of group gl, relative to gi0
-            auto grel = [&](int gl) { return static_cast<uint32_t>(((g0 + gl) >> rshift) - gi0); };
-            const uint32_t tbase = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
-                                   buf * TC_ACC_COLS + CPM * m0;
-#pragma unroll 1
-            for(int gl = 0; gl < count; gl += TR)
-            {
-                uint32_t acc[TR][C];
-                if(gl + TR <= count)
-                {
-                    // full trip: straight-line code, the folds interleave
-#pragma unroll
-                    for(int t = 0; t < TR; ++t)
-                        tmem_ld_32x32b<C>(tbase + (gl + t) * NB, acc[t]);
-                    tmem_ld_wait();
-#pragma unroll
-                    for(int t = 0; t < TR; ++t)
-                        fold(acc[t], gl + t, vb, sbyte + 2u * grel(gl + t), zbyte + grel(gl + t));
-                }
-                else
-                {
-#pragma unroll
-                    for(int t = 0; t < TR; ++t)
-                        if(gl + t < count) // the same for the whole warp
-                            tmem_ld_32x32b<C>(tbase + (gl + t) * NB, acc[t]);
-                    tmem_ld_wait();
-#pragma unroll
-                    for(int t = 0; t < TR; ++t)
-                        if(gl + t < count)
-                            fold(acc[t], gl + t, vb, sbyte + 2u * grel(gl + t), zbyte + grel(gl + t));
-                }
-            }
+            tc_fold_pass<FORM>(p, meta, vb, col, m0, tile, g0, count,
+                               tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * TC_ACC_COLS + CPM * m0, out);
             tc_fence_before_sync();
             __syncwarp();
             if(lane == 0)
@@ -650,29 +438,6 @@ __global__ void __launch_bounds__(TC_THREADS + (ESETS - 1) * 128, 1)
 // ------------------------------------------------------------------ host
 namespace {
 
-struct tc_plan
-{
-    int nb, mb, tiles, groups, blocks;
-    size_t off_sa, off_sv, total;
-};
-
-size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
-
-tc_plan make_plan(const mgx_w4_desc& d)
-{
-    tc_plan pl{};
-    // up to 8 rows: 4 int8 rows per activation row (RAW operand); up to 16: 2 rows
-    pl.nb     = d.M <= 4 ? 16 : 32;
-    pl.mb     = d.M <= 4 ? 4 : (d.M <= 8 ? 8 : 16);
-    pl.tiles  = static_cast<int>(ceil_div(d.N, TC_ROWS));
-    pl.groups = static_cast<int>(d.K / TC_GROUP_K);
-    pl.blocks = (pl.groups + TC_SUPER - 1) / TC_SUPER;
-    pl.off_sa = align_up(static_cast<size_t>(pl.nb) * d.K, 256);
-    pl.off_sv = align_up(pl.off_sa + static_cast<size_t>(pl.groups) * pl.mb * sizeof(float), 256);
-    pl.total  = pl.off_sv + static_cast<size_t>(pl.groups) * pl.mb * sizeof(int);
-    return pl;
-}
-
 // stages of the weight ring beside the planes of `items` work items
 template <int NB>
 int ring_stages(int items, int rows)
@@ -681,14 +446,14 @@ int ring_stages(int items, int rows)
     return fixed >= TC_SMEM ? 0 : static_cast<int>(std::min<size_t>(TC_MAX_STAGES, (TC_SMEM - fixed) / TC_WSTAGE));
 }
 
-template <int ESETS>
+template <class FORM>
 void configure(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2], int clusters, int split, size_t smem, cudaStream_t stream)
 {
     // programmatic dependent launch: the kernel may start while the pre-kernel still runs
     // and waits for it (griddepcontrol.wait) only where it reads what the pre-kernel wrote
     cfg                  = cudaLaunchConfig_t{};
     cfg.gridDim          = dim3(static_cast<unsigned>(clusters * split));
-    cfg.blockDim         = dim3(TC_THREADS + (ESETS - 1) * 128);
+    cfg.blockDim         = dim3(FORM::THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream           = stream;
     attr[0].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -701,7 +466,7 @@ void configure(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2], int clus
 }
 
 // Clusters of `split` CTAs that fit the device at once, one CTA per SM (asked once per kernel and device).
-template <int NB, int MR, bool RAW, int ESETS>
+template <class FORM>
 int max_clusters(int split)
 {
     static std::mutex m;
@@ -717,10 +482,10 @@ int max_clusters(int split)
     {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[2];
-        configure<ESETS>(cfg, attr, device_sm_count() / split, split, TC_SMEM, nullptr);
+        configure<FORM>(cfg, attr, device_sm_count() / split, split, TC_SMEM, nullptr);
         attr[0]      = attr[1];
         cfg.numAttrs = 1;
-        if(cudaOccupancyMaxActiveClusters(&n, w4a16_cluster_kernel<NB, MR, RAW, ESETS>, &cfg) != cudaSuccess or n < 1)
+        if(cudaOccupancyMaxActiveClusters(&n, w4a16_cluster_kernel<FORM>, &cfg) != cudaSuccess or n < 1)
         {
             (void)cudaGetLastError();
             n = device_sm_count() / (2 * split);
@@ -729,11 +494,11 @@ int max_clusters(int split)
     return n;
 }
 
-template <int NB, int MR, bool RAW, int ESETS>
+template <class FORM>
 int launch_main(int blocks, const CUtensorMap& tw, const CUtensorMap& ta, tc_params p, cudaStream_t stream)
 {
-    constexpr int rows = NB / (RAW ? 4 : 2);
-    int rc = ensure_smem_optin(reinterpret_cast<const void*>(w4a16_cluster_kernel<NB, MR, RAW, ESETS>), TC_SMEM);
+    constexpr int rows = FORM::MB;
+    int rc = ensure_smem_optin(reinterpret_cast<const void*>(w4a16_cluster_kernel<FORM>), TC_SMEM);
     if(rc != MGX_OK)
         return rc;
     // The split of K with the smallest estimated time: a CTA takes 32 KB per item at its share of the HBM
@@ -743,10 +508,10 @@ int launch_main(int blocks, const CUtensorMap& tw, const CUtensorMap& ta, tc_par
     for(int split = 1; split <= TC_MAX_SPLIT and split <= blocks; split *= 2)
     {
         const int items  = static_cast<int>(ceil_div(blocks, split));
-        const int stages = ring_stages<NB>(items, rows);
+        const int stages = ring_stages<FORM::NB>(items, rows);
         if(stages < 2)
             continue;
-        const int clusters = std::min(max_clusters<NB, MR, RAW, ESETS>(split), p.tiles);
+        const int clusters = std::min(max_clusters<FORM>(split), p.tiles);
         const int64_t mine = ceil_div(p.tiles, clusters);
         const double rate  = std::min(100.0, 6500.0 / (clusters * split));
         const double ns    = mine * items * std::max(TC_WSTAGE / rate, stages < 3 ? 1000.0 : 600.0) +
@@ -758,8 +523,8 @@ int launch_main(int blocks, const CUtensorMap& tw, const CUtensorMap& ta, tc_par
         return MGX_E_UNSUPPORTED; // (w4a16_tc_applicable says so beforehand)
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
-    configure<ESETS>(cfg, attr, p.clusters, p.split, tc_fixed<NB>(p.items, rows) + p.stages * TC_WSTAGE, stream);
-    return static_cast<int>(cudaLaunchKernelEx(&cfg, w4a16_cluster_kernel<NB, MR, RAW, ESETS>, tw, ta, p));
+    configure<FORM>(cfg, attr, p.clusters, p.split, tc_fixed<FORM::NB>(p.items, rows) + p.stages * TC_WSTAGE, stream);
+    return static_cast<int>(cudaLaunchKernelEx(&cfg, w4a16_cluster_kernel<FORM>, tw, ta, p));
 }
 
 } // namespace
@@ -774,72 +539,25 @@ bool w4a16_cluster_applicable(const mgx_w4_desc& d)
            d.K <= (d.M <= 4 ? 65536 : 28672);
 }
 
-size_t w4a16_cluster_workspace(const mgx_w4_desc& d) { return make_plan(d).total; }
+size_t w4a16_cluster_workspace(const mgx_w4_desc& d) { return tc_layout(d).end; }
 
 int w4a16_cluster_launch(const mgx_w4_desc& d, const void* A, const void* Bp, const void* scales,
                     const void* zp, void* D, void* workspace, size_t workspace_bytes,
                     cudaStream_t stream)
 {
-    const tc_plan pl = make_plan(d);
-    if(workspace == nullptr or workspace_bytes < pl.total)
+    const tc_layout lay(d);
+    if(workspace == nullptr or workspace_bytes < lay.end)
         return MGX_E_WORKSPACE;
     if((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0 or
        not w4a16_tc_pointers_ok(d, A, Bp, scales, zp))
         return MGX_E_ALIGNMENT;
-    auto* ws       = static_cast<uint8_t*>(workspace);
-    auto* aq       = reinterpret_cast<int8_t*>(ws);
-    auto* sa       = reinterpret_cast<float*>(ws + pl.off_sa);
-    auto* sv       = reinterpret_cast<int*>(ws + pl.off_sv);
     CUtensorMap tw, ta;
-    // packed weights: rows of K / 2 bytes; one request = 128 rows x 128 bytes (two groups)
-    int rc = MGX_OK;
-    {
-        cuTensorMapEncodeTiled_t encode = get_tensor_map_encoder();
-        if(encode == nullptr)
-            return MGX_E_DRIVER;
-        cuuint64_t dims[2]    = {static_cast<cuuint64_t>(d.K / 2), static_cast<cuuint64_t>(d.N)};
-        cuuint64_t strides[1] = {static_cast<cuuint64_t>(d.K / 2)};
-        cuuint32_t box[2]     = {128u, TC_ROWS};
-        cuuint32_t estr[2]    = {1u, 1u};
-        if(encode(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(Bp), dims, strides, box,
-                  estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            rc = MGX_E_INVALID_ARG;
-    }
-    if(rc != MGX_OK)
-        return rc;
-    rc = encode_grouped(&ta, aq, TC_GROUP_K, static_cast<uint64_t>(pl.nb), static_cast<uint64_t>(d.K),
-                        static_cast<uint64_t>(pl.groups), static_cast<uint32_t>(pl.nb), TC_SUPER,
-                        CU_TENSOR_MAP_SWIZZLE_128B);
-    if(rc != MGX_OK)
-        return rc;
-    rc = launch_prepare_acts(pl.mb, static_cast<const __half*>(A), d.lda, d.M, d.K, aq, sa, sv, nullptr, 0, stream);
-    if(rc != MGX_OK)
-        return rc;
     tc_params p{};
-    p.scales         = static_cast<const __half*>(scales);
-    p.zp             = static_cast<const uint8_t*>(zp);
-    p.sa             = sa;
-    p.sv             = sv;
-    p.D              = static_cast<__half*>(D);
-    p.M              = static_cast<int>(d.M);
-    p.N              = d.N;
-    p.K              = d.K;
-    p.ldd            = d.ldd;
-    p.group          = d.group;
-    p.groups_per_row = static_cast<int>(d.K / d.group);
-    p.zp_const       = d.zp_const;
-    p.tiles          = pl.tiles;
-    if(d.M == 1)
-        return launch_main<16, 1, true, 1>(pl.blocks, tw, ta, p, stream);
-    if(d.M == 2)
-        return launch_main<16, 2, true, 1>(pl.blocks, tw, ta, p, stream);
-    if(d.M <= 4)
-        return launch_main<16, 4, true, 1>(pl.blocks, tw, ta, p, stream);
-    if(d.M <= 8)
-        return launch_main<32, 8, true, 2>(pl.blocks, tw, ta, p, stream);
-    return launch_main<32, 16, false, 2>(pl.blocks, tw, ta, p, stream);
+    const int rc = tc_prepare(d, lay, A, Bp, scales, zp, D, static_cast<uint8_t*>(workspace), nullptr, 0, stream, tw, ta, p);
+    if(rc != MGX_OK)
+        return rc;
+    p.tiles = lay.tiles;
+    return tc_by_rows(d.M, [&](auto form) { return launch_main<decltype(form)>(lay.blocks, tw, ta, p, stream); });
 }
 
 int w4a16_cluster_status(unsigned int* out) { return read_and_clear_status(out); }
