@@ -243,6 +243,11 @@ def run_reference_arm(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return 0
+    from oracle import ref_target as R
+    if not R.available():
+        print(json.dumps({"impl": "reference", "unavailable": "MIGraphX's ref target (oracle/_ref) is not built: "
+                          "oracle/build_ref.py needs the MIGraphX sources"}), flush=True)
+        return 0
     r = cpu_reference(args.steps, args.warmup, 150.0)
     line = {
         "impl": "reference", "metric": METRIC, "value": r["value"], "unit": UNIT, "n_gpus": args.gpus,
