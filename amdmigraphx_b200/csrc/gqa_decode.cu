@@ -243,7 +243,9 @@ __global__ void __launch_bounds__(GD_THREADS + 32, 2)
                     continue;
                 }
                 // a sum of its own per block of 32, added in fp32: the tensor core's running sum loses a little
-                // at every step, and the score is cut to half next
+                // at every step, and the score is cut to half next.  (Of the results 0.4 to 2.8 % are not the half
+                // that the chain with 64-bit dots gives, over 14 shapes of 200 to 4096 positions; with scalar fp32
+                // sums 0.5 to 3.8 %.)
                 float cb[NB][4];
 #pragma unroll
                 for(int blk = 0; blk < NB; ++blk)

@@ -191,7 +191,9 @@ template <int V, class IndexT>
 __global__ void __launch_bounds__(256) pointwise_kernel(const __grid_constant__ pw_args a)
 {
     const mgx_pw_desc& d = a.d;
-    grid_chain();
+    if(d.insn[d.ninsns - 1].type == MGX_F16 or d.insn[d.ninsns - 1].type == MGX_F32) // (ptx.cuh)
+        grid_launch_dependents();
+    grid_dependency_wait();
     float r[MGX_PW_MAXINSN][V];
     const int last       = d.ndim - 1;
     const IndexT nvec    = static_cast<IndexT>(a.total / V);

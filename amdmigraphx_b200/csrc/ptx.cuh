@@ -211,7 +211,9 @@ __device__ __forceinline__ void grid_dependency_wait()
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// Allows the next kernel of the stream (if it was launched with the attribute) to start now.
+// Allows the next kernel of the stream (if it was launched with the attribute) to start now; without it that
+// kernel starts when this one is complete and its results can be seen.  The int4 decode linears request packed
+// weights before they wait: kernels whose results packed weights may be (8-bit integers, mgx_cuda.h) do not call it.
 __device__ __forceinline__ void grid_launch_dependents()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

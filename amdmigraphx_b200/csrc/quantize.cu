@@ -183,7 +183,9 @@ __global__ void __launch_bounds__(256)
 {
     constexpr int VEC = 16 / sizeof(In);
     constexpr bool I8 = std::is_same<Q, q_i8>::value;
-    grid_chain();
+    if constexpr(not I8) // (packed weights are 8-bit integers: ptx.cuh)
+        grid_launch_dependents();
+    grid_dependency_wait();
     const float s    = to_f32<In>(scale[0]);
     const float rcp  = static_cast<float>(1.0 / static_cast<double>(s));
     const float z    = zp == nullptr ? 0.0f : Q::zp(zp[0]);
@@ -232,7 +234,7 @@ __global__ void __launch_bounds__(256)
                     const float q0 = __fmul_rn(q[j], rcp);
                     float q1       = __fmaf_rn(__fmaf_rn(-s, q0, q[j]), rcp, q0);
                     if constexpr(not I8)
-                        q1 = copysignf(q1, q0); // the correction makes +0 of -0
+                        q1 = copysignf(q1, q0); // the correction makes +0 of -0; fp8 keeps the sign, as the other kernels here do
                     q[j] = fabsf(q0) <= 1e30f ? q1 : q0;
                     if constexpr(I8 and VEC == 8)
                         q[j] = __uint_as_float(__float_as_uint(q[j]) & 0xFFFFE000u);

@@ -30,9 +30,8 @@
 //                 in a fixed order
 // (Matrices of up to seven work items per SM take w4a16_cluster.cu, which has less around the stream; here
 // every SM streams the same number of items whatever N and K are.)
-// Launches are chained programmatically: the main kernel streams weights while the pre-kernel still runs
-// - and not while what precedes that does, which may be what writes them (the pre-kernel lets it start only
-// after its own wait; with weights requested behind that kernel's back a decoder layer took 75.0 us, 76.5 so).
+// Launches are chained programmatically: the main kernel streams weights while the pre-kernel (and the tail
+// of the previous kernel of the stream, which does not write packed weights: ptx.cuh) still runs.
 // Only plain TMA loads; every wait is bounded.
 #include "w4a16_decode.cuh"
 
@@ -171,9 +170,8 @@ __global__ void __launch_bounds__(FORM::THREADS, 1)
         // ---------------------------------------------------- TMA producer
         // A stage = 4 groups of packed weights (two requests of 128 rows x 128 bytes) + the
         // activation rows of the same groups.  The weights are requested at once: whatever
-        // wrote them is complete, the pre-kernel having waited for it before it let this kernel start.
-        // The activation rows are written by the pre-kernel, whose completion is awaited before their
-        // first request.
+        // wrote them is complete (ptx.cuh).  The activation rows are written by the pre-kernel, whose
+        // completion is awaited before their first request.
         int tile = f_lo / SG, sg = f_lo - tile * SG;
         int a_sg = sg; // the activation requests trail the weight requests at the start
         const int head = min(nsuper, WST);

@@ -10,9 +10,9 @@
  * cudaError_t reported by the CUDA runtime/driver.  Nothing throws across
  * this boundary.  There is no CPU fallback: an unsupported case is an error.
  *
- * Calls on one stream take effect in order: every operand of a call - weights, scales and
- * zero points included - may be the result of the call just before it.  (Kernels overlap with
- * their predecessor's tail, but read nothing that it may still be writing.)
+ * Calls on one stream take effect in order: an operand of a call may be the result of the call
+ * just before it.  (Kernels overlap with their predecessor's tail, but read nothing that it may
+ * still be writing.)  One operand has a condition: the packed weights of mgx_cuda_w4a16.
  *
  * Device-side problems (a bounded wait inside a kernel ran out) are recorded
  * in a per-device status word, read with mgx_cuda_device_status().
@@ -491,6 +491,13 @@ MGX_API int mgx_cuda_transpose_8bit(const void* src, void* dst, int64_t rows, in
  * fp16 out.  This is the IR parse_matmulnbits emits
  * (src/onnx/parse_matmulnbits.cpp:85-158) and what the reference fuses in
  * src/targets/gpu/fuse_mlir.cpp:1236-1276.
+ * Bp: with M <= 16 the packed weights are requested before the call waits for the work in front of it.
+ * They may be constants, or the results of earlier calls that write them as 8-bit integers (MGX_U8, MGX_I8:
+ * mgx_cuda_pointwise, _quantizelinear, ...) or as bytes (mgx_cuda_pack_int4, _copy_rows, _gather, ...), or of
+ * other kernels on the stream that do not use programmatic launch to let their successors start early: all
+ * these are complete before anything behind them starts.  They must not be the bytes of a result of another
+ * type (MGX_F16, MGX_F32, MGX_I32, MGX_FP8_E4M3FN), nor a GEMM's quantised result (mgx_qgemm_qout), of a call
+ * still in flight.  Scales and zero points have no such condition.
  * gemv: decode (M <= 16), split-K through the workspace (mgx_cuda_w4a16_workspace bytes).
  * gemm: any M (prefill); needs K % 128 == 0 and group % 128 == 0.  mgx_cuda_w4a16() picks. */
 typedef struct mgx_w4_desc
