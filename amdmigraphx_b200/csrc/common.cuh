@@ -50,12 +50,12 @@ bool w4a16_prefill_applicable(const mgx_w4_desc& d, const void* A, const void* B
 int w4a16_prefill_launch(const mgx_w4_desc& d, const void* A, const void* Bp, const void* scales,
                          const void* zp, void* D, cudaStream_t stream);
 
-// tcgen05 int4 decode path for smaller matrices (w4a16_cluster.cu)
-bool w4a16_cluster_applicable(const mgx_w4_desc& d);
-size_t w4a16_cluster_workspace(const mgx_w4_desc& d);
-int w4a16_cluster_launch(const mgx_w4_desc& d, const void* A, const void* Bp, const void* scales, const void* zp, void* D,
-                         void* workspace, size_t workspace_bytes, cudaStream_t stream);
-int w4a16_cluster_status(unsigned int* out);
+// int4 decode path for all but the largest matrices (w4a16_stream.cu); _launch gives MGX_E_UNSUPPORTED where the
+// activations do not fit in shared memory, which they do where _fits says so
+bool w4a16_stream_preferred(const mgx_w4_desc& d);
+bool w4a16_stream_fits(const mgx_w4_desc& d);
+int w4a16_stream_launch(const mgx_w4_desc& d, const void* A, const void* Bp, const void* scales, const void* zp, void* D,
+                        cudaStream_t stream);
 
 // tcgen05 int4 decode path (w4a16_tc.cu)
 bool w4a16_tc_applicable(const mgx_w4_desc& d);

@@ -119,11 +119,7 @@ extern "C" int mgx_cuda_device_status(int* status)
     rc = mgx::gqa_decode_status(&k);
     if(rc != 0)
         return rc;
-    unsigned int w = 0;
-    rc = mgx::w4a16_cluster_status(&w);
-    if(rc != 0)
-        return rc;
-    *status = static_cast<int>(w != 0 ? w : k != 0 ? k : a != 0 ? a : (b != 0 ? b : (c != 0 ? c : (d != 0 ? d : (g != 0 ? g : r)))));
+    *status = static_cast<int>(k != 0 ? k : a != 0 ? a : (b != 0 ? b : (c != 0 ? c : (d != 0 ? d : (g != 0 ? g : r)))));
     return MGX_OK;
 }
 

@@ -643,7 +643,7 @@ extern "C" size_t mgx_cuda_w4a16_workspace(const mgx_w4_desc* d)
     // pointers it is later given are 16-byte aligned
     const size_t tc = not(tc_enabled() and w4a16_tc_applicable(*d))
                           ? 0
-                          : 256 + (w4a16_cluster_applicable(*d) ? w4a16_cluster_workspace(*d) : w4a16_tc_workspace(*d));
+                          : 256 + (w4a16_stream_fits(*d) ? 0 : w4a16_tc_workspace(*d));
     if(d->M > 16 and not use_mma_path(*d))
         return tc;
     int s            = pick_splits(*d);
@@ -669,8 +669,14 @@ extern "C" int mgx_cuda_w4a16_gemv(const mgx_w4_desc* d, const void* A, const vo
         const size_t shift = workspace == nullptr ? 0 : (256 - (addr & 255u)) & 255u;
         if(workspace == nullptr or workspace_bytes < shift)
             return MGX_E_WORKSPACE;
-        auto* launch = w4a16_cluster_applicable(*d) ? w4a16_cluster_launch : w4a16_tc_launch;
-        return launch(*d, A, Bp, scales, zp, D, static_cast<uint8_t*>(workspace) + shift, workspace_bytes - shift, stream);
+        if(w4a16_stream_preferred(*d))
+        {
+            rc = w4a16_stream_launch(*d, A, Bp, scales, zp, D, stream);
+            if(rc != MGX_E_UNSUPPORTED) // (no room for the activations)
+                return rc;
+        }
+        return w4a16_tc_launch(*d, A, Bp, scales, zp, D, static_cast<uint8_t*>(workspace) + shift, workspace_bytes - shift,
+                               stream);
     }
     if(d->M > 16 and not use_mma_path(*d))
         return MGX_E_UNSUPPORTED;

@@ -1,5 +1,5 @@
-// Activations of an int4 decode linear as int8 planes: the pre-kernel both decode kernels share
-// (w4a16_tc.cu, w4a16_cluster.cu), its launch and the tensor map of its result.
+// Activations of an int4 decode linear as int8 planes: the pre-kernel of w4a16_tc.cu, its launch and the tensor map
+// of its result.
 #pragma once
 #include "common.cuh"
 #include "ptx.cuh"
