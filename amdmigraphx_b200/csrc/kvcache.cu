@@ -30,6 +30,9 @@ struct cpp_params
 template <int V> // bytes per access
 __global__ void concat_past_present_kernel(const cpp_params p)
 {
+    // (What a cache holds may be bytes of any kind, packed weights too: its successor starts when it is complete,
+    // ptx.cuh.)
+    grid_dependency_wait();
     const int64_t bh   = blockIdx.y;
     const int64_t b    = bh / p.kv_heads, h = bh % p.kv_heads;
     int64_t pos        = 0;
@@ -338,13 +341,8 @@ extern "C" int mgx_cuda_concat_past_present(const void* present, const int64_t p
     const unsigned blocks = static_cast<unsigned>(work < 256 ? 1 : (work + 255) / 256 > 1024 ? 1024 : (work + 255) / 256);
     const dim3 grid(blocks, static_cast<unsigned>(batch * kv_heads));
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-    if(v == 16)
-        concat_past_present_kernel<16><<<grid, 256, 0, stream>>>(p);
-    else if(v == 4)
-        concat_past_present_kernel<4><<<grid, 256, 0, stream>>>(p);
-    else
-        concat_past_present_kernel<1><<<grid, 256, 0, stream>>>(p);
-    return static_cast<int>(cudaGetLastError());
+    auto* kernel = v == 16 ? concat_past_present_kernel<16> : (v == 4 ? concat_past_present_kernel<4> : concat_past_present_kernel<1>);
+    return launch_dependent(kernel, grid, dim3(256), 0, stream, p);
 }
 
 extern "C" int mgx_cuda_gqa_rotary_embedding(const void* qkv, int type, int64_t batch, int64_t heads, int64_t kv_heads,

@@ -59,9 +59,8 @@ __global__ void __launch_bounds__(256) layernorm_kernel(const ln_params p)
     constexpr int TPR = 32 * WPR;       // threads per row
     __shared__ float red[2][8];
     // Without a quantised result: chained to its neighbours, so that what follows sets itself up (an int4 linear:
-    // requests its weights) while this runs (see launch_rows).
-    if(p.q == nullptr)
-        grid_launch_dependents();
+    // requests its weights) while this runs (see launch_rows) - once its own operands are requested, which would
+    // else wait behind the weights.
     grid_dependency_wait();
     const int lane    = WPR == 1 ? (threadIdx.x & 31) : threadIdx.x;
     const int64_t row = WPR == 1 ? static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)
@@ -89,6 +88,23 @@ __global__ void __launch_bounds__(256) layernorm_kernel(const ln_params p)
     const T* xr    = static_cast<const T*>(p.x) + row * p.ldx;
     float v[NV][VE];
     float sum = 0.0f;
+    // gamma and beta come with the row where there are registers for them
+    constexpr bool EARLY = NV <= 4;
+    const T* g = static_cast<const T*>(p.gamma);
+    const T* b = static_cast<const T*>(p.beta);
+    uint4 gw[EARLY ? NV : 1], bw[EARLY ? NV : 1];
+    if constexpr(EARLY)
+    {
+#pragma unroll
+        for(int i = 0; i < NV; ++i)
+        {
+            const int vi = lane + TPR * i;
+            if(g != nullptr and vi < nvec)
+                gw[i] = *reinterpret_cast<const uint4*>(g + vi * VE);
+            if(b != nullptr and vi < nvec)
+                bw[i] = *reinterpret_cast<const uint4*>(b + vi * VE);
+        }
+    }
 #pragma unroll
     for(int i = 0; i < NV; ++i)
     {
@@ -123,8 +139,11 @@ __global__ void __launch_bounds__(256) layernorm_kernel(const ln_params p)
                 v[i][j] = 0.0f;
         }
     }
-    sum = row_sum(sum, 0);
-    const float mean = ln_round<T>(sum * p.inv_n);
+    if(p.q == nullptr)
+        grid_launch_dependents();
+    float mean = 0.0f;
+    if(not p.rms)
+        mean = ln_round<T>(row_sum(sum, 0) * p.inv_n);
     float sq = 0.0f;
     if(p.rms)
     {
@@ -160,8 +179,6 @@ __global__ void __launch_bounds__(256) layernorm_kernel(const ln_params p)
     const float ve  = ln_round<T>(var + p.eps);
     // rsqrt as the reference computes it: 1 / sqrt(x), both correctly rounded in fp32
     const float rs  = ln_round<T>(__fdiv_rn(1.0f, __fsqrt_rn(ve)));
-    const T* g = static_cast<const T*>(p.gamma);
-    const T* b = static_cast<const T*>(p.beta);
     const float q_lo = -128.0f - p.q_zp, q_hi = 127.0f - p.q_zp;
 #pragma unroll
     for(int i = 0; i < NV; ++i)
@@ -172,7 +189,7 @@ __global__ void __launch_bounds__(256) layernorm_kernel(const ln_params p)
         float gv[VE], bv[VE];
         if(g != nullptr)
         {
-            const uint4 w = __ldg(reinterpret_cast<const uint4*>(g + vi * VE));
+            const uint4 w = EARLY ? gw[EARLY ? i : 0] : *reinterpret_cast<const uint4*>(g + vi * VE);
             if constexpr(std::is_same<T, float>::value)
                 gv[0] = __uint_as_float(w.x), gv[1] = __uint_as_float(w.y), gv[2] = __uint_as_float(w.z),
                 gv[3] = __uint_as_float(w.w);
@@ -189,7 +206,7 @@ __global__ void __launch_bounds__(256) layernorm_kernel(const ln_params p)
         }
         if(b != nullptr)
         {
-            const uint4 w = __ldg(reinterpret_cast<const uint4*>(b + vi * VE));
+            const uint4 w = EARLY ? bw[EARLY ? i : 0] : *reinterpret_cast<const uint4*>(b + vi * VE);
             if constexpr(std::is_same<T, float>::value)
                 bv[0] = __uint_as_float(w.x), bv[1] = __uint_as_float(w.y), bv[2] = __uint_as_float(w.z),
                 bv[3] = __uint_as_float(w.w);

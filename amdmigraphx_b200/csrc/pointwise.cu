@@ -402,13 +402,17 @@ enum { PW_FORM_BINARY, PW_FORM_SWIGLU };
 template <int FORM>
 __global__ void __launch_bounds__(256) pointwise_f16_kernel(const pw_f16_args a)
 {
+    // Its successor may start when the operands are requested: an int4 decode linear then requests its weights
+    // behind them and not in front of them.
+    grid_dependency_wait();
     const uint32_t nvec = a.rows * a.row_vecs;
     for(uint32_t vec = blockIdx.x * 256u + threadIdx.x; vec < nvec; vec += gridDim.x * 256u)
     {
-        const uint32_t row = vec / a.row_vecs, col = vec - row * a.row_vecs;
+        const uint32_t row = a.rows == 1 ? 0u : vec / a.row_vecs, col = vec - row * a.row_vecs;
         float x[8], y[8], r[8];
         pw_load_vec<8>(a.in0, MGX_F16, row * a.stride0 + col * 8, 1, x);
         pw_load_vec<8>(a.in1, MGX_F16, row * a.stride1 + col * 8, 1, y);
+        grid_launch_dependents();
         if constexpr(FORM == PW_FORM_BINARY)
         {
 #pragma unroll
@@ -482,11 +486,8 @@ static bool launch_pointwise_f16_form(const pw_args& a, cudaStream_t stream, int
     const int64_t blocks = ceil_div(a.total / 8, 256);
     const int64_t cap    = static_cast<int64_t>(device_sm_count()) * 8;
     const int grid       = static_cast<int>(blocks < cap ? blocks : cap);
-    if(form == PW_FORM_BINARY)
-        pointwise_f16_kernel<PW_FORM_BINARY><<<grid, 256, 0, stream>>>(f);
-    else
-        pointwise_f16_kernel<PW_FORM_SWIGLU><<<grid, 256, 0, stream>>>(f);
-    status = static_cast<int>(cudaGetLastError());
+    status = launch_dependent(form == PW_FORM_BINARY ? pointwise_f16_kernel<PW_FORM_BINARY> : pointwise_f16_kernel<PW_FORM_SWIGLU>,
+                              dim3(static_cast<unsigned>(grid)), dim3(256), 0, stream, f);
     return true;
 }
 
