@@ -35,6 +35,7 @@ constexpr int GD_THREADS    = 32 * GD_WARPS; // consumers; one more warp request
 constexpr int GD_TILE       = 64;            // positions
 constexpr int GD_HEADS      = 8;             // query heads per KV head, padded
 constexpr int GD_MAX_STAGES = 12;
+constexpr int GD_MAX_SPLIT  = 8;
 
 struct gqa_decode_params
 {
@@ -47,7 +48,7 @@ struct gqa_decode_params
     float scale;
     int cache_seq, kv_heads, fact;
     int jobs, split; // (batch entry, KV head) pairs; CTAs of a cluster
-    int cap, stages; // score columns a CTA holds in shared memory; tiles of its ring
+    int cap, pitch, stages; // score columns a CTA holds in shared memory; tiles of its ring
 };
 
 __device__ __forceinline__ float gd_exp2(float x)
@@ -127,8 +128,9 @@ __global__ void __launch_bounds__(GD_THREADS + 32, 2)
         fence_barrier_init();
     }
     __syncthreads();
+    // the other CTAs' barriers exist before anyone arrives on them: waited for at the first exchange
     if(p.split > 1)
-        cluster_barrier(); // the other CTAs' barriers exist before anyone arrives on them
+        cluster_barrier_arrive();
     const int rank  = static_cast<int>(blockIdx.x) % p.split;
     const int first = static_cast<int>(blockIdx.x) / p.split, step = static_cast<int>(gridDim.x) / p.split;
     grid_dependency_wait(); // caches, queries and lengths may come from the previous kernel
@@ -169,6 +171,8 @@ __global__ void __launch_bounds__(GD_THREADS + 32, 2)
                     s = 0, ph ^= 1;
             }
         }
+        if(p.split > 1)
+            cluster_barrier_wait();
     }
     else
     {
@@ -185,12 +189,28 @@ __global__ void __launch_bounds__(GD_THREADS + 32, 2)
             gd_consumer_barrier();
             if(p.split > 1)
             {
+                if(xch == 0)
+                    cluster_barrier_wait();
                 if(tid < p.split)
                     cluster_arrive(&peer_bar, tid);
                 if(not dead and not __all_sync(0xffffffffu, mbar_wait_cluster_bounded(&peer_bar, xch & 1, abort_flag, 6)))
                     dead = true;
             }
             ++xch;
+        };
+        // what the CTAs of the cluster hold at `at`, added in their order, or the largest: all under way together (one
+        // after another 0.2 us each)
+        auto of_cluster = [&](const float* at, bool largest) {
+            float v[GD_MAX_SPLIT];
+#pragma unroll
+            for(int r = 0; r < GD_MAX_SPLIT; ++r)
+                v[r] = __uint_as_float(cluster_load(at, min(r, p.split - 1)));
+            float x = v[0];
+#pragma unroll
+            for(int r = 1; r < GD_MAX_SPLIT; ++r)
+                if(r < p.split)
+                    x = largest ? fmaxf(x, v[r]) : x + v[r];
+            return x;
         };
         auto wait_tile = [&](int tile) {
             if(not dead and not mbar_wait_warp(&full_bar[tile % p.stages], (tile / p.stages) & 1, abort_flag, 1))
@@ -270,7 +290,7 @@ __global__ void __launch_bounds__(GD_THREADS + 32, 2)
                         float sv = truncate_to_half_precision(c);
                         sv       = truncate_to_half_precision(__fmul_rn(sv, p.scale));
                         mx[e & 1]          = fmaxf(mx[e & 1], sv);
-                        sc[h * p.cap + j] = __float2half_rz(sv);
+                        sc[h * p.pitch + j] = __float2half_rz(sv);
                     }
                 }
             }
@@ -296,52 +316,42 @@ __global__ void __launch_bounds__(GD_THREADS + 32, 2)
             if(p.split > 1)
             {
                 if(tid < GD_HEADS)
-                {
-                    float m = -INFINITY;
-                    for(int r = 0; r < p.split; ++r)
-                        m = fmaxf(m, __uint_as_float(cluster_load(red_m + tid, r)));
-                    tot_m[tid] = m;
-                }
+                    tot_m[tid] = of_cluster(red_m + tid, true);
                 gd_consumer_barrier();
             }
             const float* gmax = p.split > 1 ? tot_m : red_m;
-            // ---- e = half(exp(x - max)) in place, the sum over the stored halves in fp32
-            for(int h = 0; h < p.fact; ++h)
+            // ---- e = half(exp(x - max)) in place, the sum over the stored halves in fp32; 8 / fact warps a head
             {
-                const float gm = gmax[h];
-                float s        = 0.0f;
-                for(int j = tid; j < n; j += GD_THREADS)
+                const int parts = GD_WARPS / p.fact, h = warp / parts;
+                const float gm  = gmax[h];
+                float s         = 0.0f;
+                for(int j = (warp - h * parts) * 32 + lane; j < n; j += 32 * parts)
                 {
-                    const float x = __half2float(sc[h * p.cap + j]);
+                    const float x = __half2float(sc[h * p.pitch + j]);
                     const float e = gd_trunc_nonneg(gd_exp2((x - gm) * log2e));
-                    sc[h * p.cap + j] = __float2half_rz(e);
+                    sc[h * p.pitch + j] = __float2half_rz(e);
                     s += e;
                 }
 #pragma unroll
                 for(int o = 16; o > 0; o >>= 1)
                     s += __shfl_xor_sync(0xffffffffu, s, o);
                 if(lane == 0)
-                    wred[warp][h] = s; // (the maxima in wred were read before the exchange)
+                    wred[warp][0] = s; // (the maxima in wred were read before the exchange)
             }
             gd_consumer_barrier();
             if(tid < p.fact)
             {
-                float s = 0.0f;
-#pragma unroll
-                for(int w = 0; w < GD_WARPS; ++w)
-                    s += wred[w][tid];
+                const int parts = GD_WARPS / p.fact;
+                float s         = 0.0f;
+                for(int w = 0; w < parts; ++w)
+                    s += wred[tid * parts + w][0];
                 red_s[tid] = s;
             }
             exchange();
             if(p.split > 1)
             {
                 if(tid < p.fact)
-                {
-                    float s = 0.0f;
-                    for(int r = 0; r < p.split; ++r)
-                        s += __uint_as_float(cluster_load(red_s + tid, r));
-                    tot_s[tid] = s;
-                }
+                    tot_s[tid] = of_cluster(red_s + tid, false);
                 gd_consumer_barrier();
             }
             // ---- partial P V: p = half(e / sum) where it is used (one reciprocal per head, the quotient
@@ -369,7 +379,7 @@ __global__ void __launch_bounds__(GD_THREADS + 32, 2)
                     for(int i = 0; i < 2; ++i)
                     {
                         const int j      = j0 + 8 * i + 2 * t;
-                        const uint32_t w = *reinterpret_cast<const uint32_t*>(sc + g * p.cap + j);
+                        const uint32_t w = *reinterpret_cast<const uint32_t*>(sc + g * p.pitch + j);
                         const float2 e2  = __half22float2(*reinterpret_cast<const __half2*>(&w));
                         float a0 = e2.x * rcp, a1 = e2.y * rcp;
                         a0 = __fmaf_rn(__fmaf_rn(-a0, total, e2.x), rcp, a0);
@@ -420,12 +430,7 @@ __global__ void __launch_bounds__(GD_THREADS + 32, 2)
             exchange();
             if(p.split > 1)
                 for(int i = tid + rank * GD_THREADS; i < p.fact * D; i += p.split * GD_THREADS)
-                {
-                    float s = 0.0f;
-                    for(int r = 0; r < p.split; ++r)
-                        s += __uint_as_float(cluster_load(cta_out + i, r));
-                    dst[i] = __float2half_rz(s);
-                }
+                    dst[i] = __float2half_rz(of_cluster(cta_out + i, false));
         }
     }
     // ---------------------------------------------------------- teardown
@@ -441,12 +446,13 @@ __global__ void __launch_bounds__(GD_THREADS + 32, 2)
 namespace {
 
 // dynamic shared memory of a CTA when `resident` of them share an SM (beside the static arrays)
-constexpr size_t smem_max(int resident) { return (resident == 1 ? 220 : 106) * 1024; }
+constexpr size_t smem_max(int resident) { return (resident == 1 ? 220 : 106) * 1024 + 128; }
 
-// Bytes of the score / partial-result region for a share of `cap` positions.
+// Bytes of the score / partial-result region for a share of `cap` positions (a multiple of 16).  The heads' rows are
+// cap + 8 halves apart: an odd multiple of 16 bytes, so that eight heads' words lie in different banks.
 size_t region_bytes(int64_t fact, int64_t head, int64_t cap)
 {
-    return std::max<size_t>(sizeof(__half) * fact * cap, sizeof(float) * GD_WARPS * fact * head);
+    return std::max<size_t>(sizeof(__half) * fact * (cap + 8), sizeof(float) * GD_WARPS * fact * head);
 }
 
 int64_t share_cap(int64_t cache_seq, int split) { return (ceil_div(cache_seq, split) + 15) / 16 * 16; }
@@ -530,6 +536,7 @@ int launch_gqa_decode(gqa_decode_params p, const void* k_cache, const void* v_ca
     if(best == 0.0)
         return MGX_E_TOO_LARGE;
     const size_t region = region_bytes(p.fact, D, p.cap);
+    p.pitch             = p.cap + 8;
     p.stages = static_cast<int>(std::min<size_t>(GD_MAX_STAGES, (smem_max(per_sm) - 1024 - region) / (GD_TILE * D * 2)));
     CUtensorMap tk, tv;
     cuTensorMapEncodeTiled_t encode = get_tensor_map_encoder();
