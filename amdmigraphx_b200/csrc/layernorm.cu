@@ -58,9 +58,8 @@ __global__ void __launch_bounds__(256) layernorm_kernel(const ln_params p)
     constexpr int VE  = 16 / sizeof(T); // elements per vector
     constexpr int TPR = 32 * WPR;       // threads per row
     __shared__ float red[2][8];
-    // Without a quantised result: chained to its neighbours, so that what follows sets itself up (an int4 linear:
-    // requests its weights) while this runs (see launch_rows) - once its own operands are requested, which would
-    // else wait behind the weights.
+    // Chained to its neighbours; what follows sets itself up (an int4 linear: requests its weights) while this runs
+    // (see launch_rows) - once this row's operands are requested, which would else wait behind the weights.
     grid_dependency_wait();
     const int lane    = WPR == 1 ? (threadIdx.x & 31) : threadIdx.x;
     const int64_t row = WPR == 1 ? static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)
@@ -287,16 +286,14 @@ __global__ void __launch_bounds__(256) layernorm_kernel(const ln_params p)
     }
 }
 
-// 256 threads a block.  A norm without a quantised result (a decoder layer's) is launched programmatically: an int4
-// decode linear behind it begins 2 us earlier (one row, norm and linear back to back: 4096 x 4096 10.2 -> 8.0 us,
-// 12288 x 4096 12.3 -> 10.4).  One with a quantised result is not: an int8 result may be packed weights (ptx.cuh), so
-// its successor cannot start early, and its own early start costs the encoder's layer of 3072 rows 1.9 of 106 us.
+// 256 threads a block, launched programmatically: a layer's norm starts 1 to 2 us earlier behind a GEMM (encoder layer
+// of 985 rows, launched one by one, 63.0 -> 58.5 us; of 3072 rows in a graph 105.4 -> 104.8).  What follows may start
+// early too unless the result is quantised: an int8 result may be packed weights (ptx.cuh).  An int4 decode linear
+// behind an RMSNorm then begins 2 us earlier (one row, norm and linear back to back: 4096 x 4096 10.2 -> 8.0 us,
+// 12288 x 4096 12.3 -> 10.4).
 static int launch_rows(void (*kernel)(ln_params), dim3 grid, const ln_params& p, cudaStream_t stream)
 {
-    if(p.q == nullptr)
-        return launch_dependent(kernel, grid, dim3(256), 0, stream, p);
-    kernel<<<grid, 256, 0, stream>>>(p);
-    return static_cast<int>(cudaGetLastError());
+    return launch_dependent(kernel, grid, dim3(256), 0, stream, p);
 }
 
 template <class T>
