@@ -70,6 +70,18 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void* smem)
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(s));
 }
+__device__ __forceinline__ void ldmatrix_x4_at(uint32_t (&r)[4], uint32_t s)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(s));
+}
+__device__ __forceinline__ void ldmatrix_x4_trans_at(uint32_t (&r)[4], uint32_t s)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(s));
+}
 __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void* smem)
 {
     const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
@@ -85,6 +97,15 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4],
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// The same with nothing to add to.
+__device__ __forceinline__ void mma_16816_first(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
+{
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+                 "{%8, %9}, {%10, %10, %10, %10};"
+                 : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
+}
+
 // 2^x for x <= 0 (and -inf-like arguments, which give 0): one instruction
 __device__ __forceinline__ float fast_exp2(float x)
 {
@@ -92,6 +113,36 @@ __device__ __forceinline__ float fast_exp2(float x)
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+
+// Two fp32 operations as one instruction, each rounded as by itself.
+__device__ __forceinline__ float2 add2(float2 a, float2 b)
+{
+    float2 d;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 z, x, y;\n\t"
+        "mov.b64 {%0, %1}, z;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b)
+{
+    float2 d;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 z, x, y;\n\t"
+        "mov.b64 {%0, %1}, z;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
+{
+    float2 d;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+        "fma.rn.f32x2 z, x, y, z;\n\tmov.b64 {%0, %1}, z;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
 
 // A [rows, 64] fp16 tile in shared memory: 128-byte rows, the 16-byte chunk index XOR-ed with the
 // row's low three bits.
@@ -296,7 +347,7 @@ __global__ void __launch_bounds__(128) attention_f16_kernel(const attention_para
 
 // ---------------------------------------------------------------------------------------------
 // The operator chain's own roundings (see the head of the file).  Dynamic shared memory:
-// Q tile | two K / V tiles | scores [64][sp] half (sp = keys rounded up to 64, + 8 against bank
+// three K / V tiles | scores [64][sp] half (first the Q tile) (sp = keys rounded up to 64, + 8 against bank
 // conflicts) | row maxima.
 constexpr int AT_CHAIN_MAX_SEQ = 1024;
 
@@ -311,13 +362,14 @@ __device__ __forceinline__ float trunc_half_nonneg(float v)
 
 constexpr int ATC_THREADS = 256;
 
-// load_tile for a block of ATC_THREADS threads
+// ROWS x 64 halves by a block of ATC_THREADS threads
+template <int ROWS>
 __device__ __forceinline__ void load_tile_256(__half* tile, const __half* g, int64_t ld, int rows_left, int tid)
 {
 #pragma unroll
-    for(int i = 0; i < 2; ++i)
+    for(int i = 0; i < ROWS * 8 / ATC_THREADS; ++i)
     {
-        const int c   = tid + i * ATC_THREADS; // 512 chunks of 16 bytes
+        const int c   = tid + i * ATC_THREADS; // chunks of 16 bytes
         const int row = c >> 3, chunk = c & 7;
         const bool ok = row < rows_left;
         cp_async_16(tile_ptr(tile, row, chunk), g + (ok ? row : 0) * ld + chunk * 8, ok);
@@ -329,8 +381,8 @@ __device__ __forceinline__ void load_tile_256(__half* tile, const __half* g, int
 // through shared memory at the end); in the softmax phase every warp owns 8 whole rows.  Twice the
 // warps of one-warp-per-16-rows at half the accumulator registers each: the kernel is bound by
 // the latency of dependent instructions, which only more resident warps hide.
-// NVMAX: half2 pairs per lane and row the softmax phase holds in registers (keys <= 64 NVMAX).
-template <int NVMAX, int RG>
+// NV: tiles of 64 keys = half2 pairs per lane and row that the softmax phase holds in registers.
+template <int NV, int RG>
 __global__ void __launch_bounds__(ATC_THREADS, 3) attention_f16_chain_kernel(const attention_params p, const int sp)
 {
     constexpr int BMC = RG * 16;      // query rows per CTA
@@ -338,9 +390,8 @@ __global__ void __launch_bounds__(ATC_THREADS, 3) attention_f16_chain_kernel(con
     constexpr int JPW = 4 / KS;       // 16-key groups of a tile per warp
     constexpr int RPW = BMC / 8;      // whole rows per warp in the softmax phase
     extern __shared__ __align__(128) uint8_t at_smem[];
-    __half* sq     = reinterpret_cast<__half*>(at_smem);
-    __half* skv[2] = {sq + AT_BM * AT_D, sq + AT_BM * AT_D + AT_BN * AT_D};
-    __half* sc     = sq + AT_BM * AT_D + 2 * AT_BN * AT_D; // [BMC][sp]
+    __half* skv    = reinterpret_cast<__half*>(at_smem); // three tiles
+    __half* sc     = skv + 3 * AT_BN * AT_D;             // [BMC][sp]; the query rows until the first scores
     float* rowmax  = reinterpret_cast<float*>(sc + BMC * sp); // [KS][BMC]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, t = lane & 3;
@@ -351,11 +402,53 @@ __global__ void __launch_bounds__(ATC_THREADS, 3) attention_f16_chain_kernel(con
     const __half* qg = p.q + (row_base + q0) * p.ldq + head * AT_D;
     const __half* kg = p.k + row_base * p.ldk + head * AT_D;
     const __half* vg = p.v + row_base * p.ldv + head * AT_D;
-    const int nblocks = (p.seq + AT_BN - 1) / AT_BN;
-
-    load_tile_256(sq, qg, p.ldq, p.seq - q0, tid);
-    load_tile_256(skv[0], kg, p.ldk, p.seq, tid);
-    cp_async_commit();
+    // The tiles of K, then those of V, go round three places, two ahead of the one in use: a tile travels for about
+    // as long as two take.  (8 x 384 tokens, 12 heads: one ahead 34.3 us, two 32.9; with addresses that advance instead
+    // of being worked out per tile, the number of tiles known and packed fp32 arithmetic 29.1.  What is left is latency:
+    // four and a half warps to a scheduler, the second wave of CTAs 30 % full.)
+    // This thread's part of a tile: 16 bytes of rows tid / 8 and tid / 8 + 32.
+    const int l_row       = tid >> 3;
+    const uint32_t l_at   = smem_u32(tile_ptr(skv, l_row, tid & 7)); // (rows 32 apart have the same swizzle)
+    const __half* l_k     = kg + l_row * p.ldk + (tid & 7) * 8;
+    const __half* l_v     = vg + l_row * p.ldv + (tid & 7) * 8;
+    int l_u = 0, l_place = 0, l_left = p.seq - l_row; // tile to request, its place, rows of it from l_row on
+    auto request = [&] {
+        if(l_u < 2 * NV)
+        {
+            const __half*& src = l_u < NV ? l_k : l_v;
+            const int64_t ld   = l_u < NV ? p.ldk : p.ldv;
+#pragma unroll
+            for(int i = 0; i < 2; ++i)
+            {
+                // (a row beyond the sequence: nothing is read, the address is that of one which is there)
+                const bool ok = l_left > 32 * i;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(l_at + l_place * (AT_BN * AT_D * 2) + i * 4096),
+                             "l"(ok ? src + i * 32 * ld : qg), "r"(ok ? 16 : 0)
+                             : "memory");
+            }
+            src += 64 * ld;
+            l_left -= 64;
+            if(++l_place == 3)
+                l_place = 0;
+            if(++l_u == NV)
+                l_left = p.seq - l_row;
+        }
+        cp_async_commit();
+    };
+    load_tile_256<BMC>(sc, qg, p.ldq, p.seq - q0, tid);
+    request();
+    request();
+    // ldmatrix addresses: row and chunk of a tile for k-step ks are this thread's; 16 rows on are 2 KB on
+    const int lr       = (lane & 7) + ((lane >> 3) & 1) * 8;
+    const int kr       = (lane & 7) + (lane >> 4) * 8;
+    uint32_t k_off[4], v_off[4];
+#pragma unroll
+    for(int i = 0; i < 4; ++i)
+    {
+        k_off[i] = kr * 128 + (((2 * i + ((lane >> 3) & 1)) ^ (kr & 7)) << 4);
+        v_off[i] = lr * 128 + (((2 * i + (lane >> 4)) ^ (lr & 7)) << 4);
+    }
+    const uint32_t tiles = smem_u32(skv);
 
     // ---- phase 1: scores = half(half(Q K^T) * scale) into shared memory, row maxima
     {
@@ -364,29 +457,21 @@ __global__ void __launch_bounds__(ATC_THREADS, 3) attention_f16_chain_kernel(con
         // keys} of row g + 8 r
         const __half2 lowest = __floats2half2_rn(-65504.0f, -65504.0f);
         __half2 mxh[2]       = {lowest, lowest};
-        for(int kb = 0; kb < nblocks; ++kb)
+#pragma unroll 1
+        for(int kb = 0; kb < NV; ++kb)
         {
-            const int buf = kb & 1;
-            if(kb + 1 < nblocks)
-            {
-                const int k1 = (kb + 1) * AT_BN;
-                load_tile_256(skv[buf ^ 1], kg + static_cast<int64_t>(k1) * p.ldk, p.ldk, p.seq - k1, tid);
-                cp_async_commit();
-                cp_async_wait<1>();
-            }
-            else
-                cp_async_wait<0>();
-            __syncthreads();
+            cp_async_wait<1>();
+            __syncthreads(); // tile kb is there, everyone is done with the one before
+            request();
+            const uint32_t tile = tiles + kb % 3 * (AT_BN * AT_D * 2) + kh * (JPW * 2048);
             if(kb == 0)
             {
 #pragma unroll
                 for(int ks = 0; ks < 4; ++ks)
-                    ldmatrix_x4(qa[ks], tile_ptr(sq, rg * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, 2 * ks + (lane >> 4)));
+                    ldmatrix_x4(qa[ks], tile_ptr(sc, rg * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, 2 * ks + (lane >> 4)));
+                __syncthreads(); // the scores take the query rows' place
             }
             float s[2 * JPW][4];
-#pragma unroll
-            for(int j = 0; j < 2 * JPW; ++j)
-                s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.0f;
 #pragma unroll
             for(int ks = 0; ks < 4; ++ks)
             {
@@ -394,44 +479,58 @@ __global__ void __launch_bounds__(ATC_THREADS, 3) attention_f16_chain_kernel(con
                 for(int jp = 0; jp < JPW; ++jp)
                 {
                     uint32_t kf[4];
-                    ldmatrix_x4(kf, tile_ptr(skv[buf], (kh * JPW + jp) * 16 + (lane & 7) + (lane >> 4) * 8,
-                                             2 * ks + ((lane >> 3) & 1)));
+                    ldmatrix_x4_at(kf, tile + jp * 2048 + k_off[ks]);
+                    if(ks == 0)
+                    {
+                        mma_16816_first(s[2 * jp], qa[ks], kf[0], kf[1]);
+                        mma_16816_first(s[2 * jp + 1], qa[ks], kf[2], kf[3]);
+                        continue;
+                    }
                     mma_16816(s[2 * jp], qa[ks], kf[0], kf[1]);
                     mma_16816(s[2 * jp + 1], qa[ks], kf[2], kf[3]);
                 }
             }
             const int kbase = kb * AT_BN + kh * (16 * JPW);
-            const bool tail = kbase + 16 * JPW > p.seq;
+            const bool tail = kb == NV - 1 and kbase + 16 * JPW > p.seq;
             // half(Q K^T): mantissa cut (a score in the half subnormal range keeps a few more bits:
             // below 2^-24 absolute, invisible after the exponential); half(score * scale): the
             // packing conversion itself rounds toward zero, subnormal halves included
+            uint32_t w[2 * JPW][2];
+#pragma unroll
+            for(int j = 0; j < 2 * JPW; ++j)
+#pragma unroll
+                for(int r = 0; r < 2; ++r)
+                {
+                    const float2 x = mul2(make_float2(__uint_as_float(__float_as_uint(s[j][2 * r]) & 0xFFFFE000u),
+                                                      __uint_as_float(__float_as_uint(s[j][2 * r + 1]) & 0xFFFFE000u)),
+                                          both(p.scale));
+                    w[j][r]        = cvt_rz_f16x2(x.x, x.y);
+                }
+            // keys that do not exist: the lowest half, whose exponential is 0 (a loop, or the compiler does it for
+            // every tile)
+#pragma unroll 1
+            for(int once = tail ? 1 : 0; once > 0; --once)
+            {
+#pragma unroll
+                for(int j = 0; j < 2 * JPW; ++j)
+                {
+                    const int left      = p.seq - (kbase + j * 8 + 2 * t);
+                    const uint32_t keep = left > 1 ? 0xFFFFFFFFu : (left == 1 ? 0x0000FFFFu : 0u);
+#pragma unroll
+                    for(int r = 0; r < 2; ++r)
+                        w[j][r] = (w[j][r] & keep) | (0xFBFFFBFFu & ~keep);
+                }
+            }
 #pragma unroll
             for(int j = 0; j < 2 * JPW; ++j)
             {
-                float x[4];
-#pragma unroll
-                for(int e = 0; e < 4; ++e)
-                    x[e] = __uint_as_float(__float_as_uint(s[j][e]) & 0xFFFFE000u) * p.scale;
-                if(tail)
-                {
-                    // keys that do not exist: the lowest half, whose exponential is 0
-#pragma unroll
-                    for(int e = 0; e < 4; ++e)
-                        if(kbase + j * 8 + 2 * t + (e & 1) >= p.seq)
-                            x[e] = -65504.0f;
-                }
-                const uint32_t w0 = cvt_rz_f16x2(x[0], x[1]), w1 = cvt_rz_f16x2(x[2], x[3]);
-                mxh[0]            = __hmax2(mxh[0], *reinterpret_cast<const __half2*>(&w0));
-                mxh[1]            = __hmax2(mxh[1], *reinterpret_cast<const __half2*>(&w1));
-                const int col     = kbase + j * 8 + 2 * t;
-                *reinterpret_cast<uint32_t*>(sc + (rg * 16 + g) * sp + col)     = w0;
-                *reinterpret_cast<uint32_t*>(sc + (rg * 16 + g + 8) * sp + col) = w1;
+                mxh[0]        = __hmax2(mxh[0], *reinterpret_cast<const __half2*>(&w[j][0]));
+                mxh[1]        = __hmax2(mxh[1], *reinterpret_cast<const __half2*>(&w[j][1]));
+                const int col = kbase + j * 8 + 2 * t;
+                *reinterpret_cast<uint32_t*>(sc + (rg * 16 + g) * sp + col)     = w[j][0];
+                *reinterpret_cast<uint32_t*>(sc + (rg * 16 + g + 8) * sp + col) = w[j][1];
             }
-            __syncthreads(); // the other tile is overwritten by the next iteration's load
         }
-        // V's first tile travels while the softmax runs
-        load_tile_256(skv[0], vg, p.ldv, p.seq, tid);
-        cp_async_commit();
 #pragma unroll
         for(int r = 0; r < 2; ++r)
         {
@@ -450,7 +549,6 @@ __global__ void __launch_bounds__(ATC_THREADS, 3) attention_f16_chain_kernel(con
     // against the 5e-4 spacing of the halves it is truncated to), the quotient from one reciprocal
     // per row and a remainder correction (correctly rounded before the truncation).
     {
-        const int nv = nblocks; // half2 pairs per lane and row: keys / 64
         constexpr float log2e = 1.4426950408889634f;
 #pragma unroll 1
         for(int r = 0; r < RPW; ++r)
@@ -463,32 +561,30 @@ __global__ void __launch_bounds__(ATC_THREADS, 3) attention_f16_chain_kernel(con
                 m = fmaxf(m, rowmax[h * BMC + row]);
             // the packing conversion rounds toward zero (subnormal halves included); the sum runs
             // over the stored halves
-            float2 e[NVMAX];
-            float sum = 0.0f;
+            float2 e[NV], sums = both(0.0f);
 #pragma unroll
-            for(int i = 0; i < NVMAX; ++i)
+            for(int i = 0; i < NV; ++i)
             {
-                if(i < nv)
                 {
                     const float2 x   = __half22float2(*reinterpret_cast<const __half2*>(rowp + i * 64 + lane * 2));
-                    const uint32_t h = cvt_rz_f16x2(fast_exp2((x.x - m) * log2e), fast_exp2((x.y - m) * log2e));
+                    const float2 y   = mul2(add2(x, both(-m)), both(log2e));
+                    const uint32_t h = cvt_rz_f16x2(fast_exp2(y.x), fast_exp2(y.y));
                     e[i]             = __half22float2(*reinterpret_cast<const __half2*>(&h));
-                    sum += e[i].x + e[i].y;
+                    sums             = add2(sums, e[i]);
                 }
             }
+            float sum = sums.x + sums.y;
 #pragma unroll
             for(int o = 16; o > 0; o >>= 1)
                 sum += __shfl_xor_sync(0xffffffffu, sum, o);
             const float rcp = __frcp_rn(sum);
 #pragma unroll
-            for(int i = 0; i < NVMAX; ++i)
+            for(int i = 0; i < NV; ++i)
             {
-                if(i < nv)
                 {
-                    float a = e[i].x * rcp, b = e[i].y * rcp;
-                    a       = __fmaf_rn(__fmaf_rn(-a, sum, e[i].x), rcp, a);
-                    b       = __fmaf_rn(__fmaf_rn(-b, sum, e[i].y), rcp, b);
-                    *reinterpret_cast<uint32_t*>(rowp + i * 64 + lane * 2) = cvt_rz_f16x2(a, b);
+                    const float2 a = mul2(e[i], both(rcp));
+                    const float2 b = fma2(fma2(a, both(-sum), e[i]), both(rcp), a);
+                    *reinterpret_cast<uint32_t*>(rowp + i * 64 + lane * 2) = cvt_rz_f16x2(b.x, b.y);
                 }
             }
         }
@@ -497,41 +593,35 @@ __global__ void __launch_bounds__(ATC_THREADS, 3) attention_f16_chain_kernel(con
 
     // ---- phase 3: O = P V with the half probabilities as A fragments straight from shared
     // memory; this warp's half of every tile's keys
+    const uint32_t p_at = smem_u32(sc + (rg * 16 + lr) * sp + (lane >> 4) * 8);
     float o[8][4];
 #pragma unroll
     for(int j = 0; j < 8; ++j)
         o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.0f;
-    for(int kb = 0; kb < nblocks; ++kb)
+#pragma unroll 1
+    for(int kb = 0; kb < NV; ++kb)
     {
-        const int buf = kb & 1;
-        if(kb + 1 < nblocks)
-        {
-            const int k1 = (kb + 1) * AT_BN;
-            load_tile_256(skv[buf ^ 1], vg + static_cast<int64_t>(k1) * p.ldv, p.ldv, p.seq - k1, tid);
-            cp_async_commit();
-            cp_async_wait<1>();
-        }
-        else
-            cp_async_wait<0>();
+        cp_async_wait<1>();
         __syncthreads();
+        request();
+        const uint32_t tile = tiles + (NV + kb) % 3 * (AT_BN * AT_D * 2);
 #pragma unroll
         for(int k2 = 0; k2 < JPW; ++k2)
         {
             const int ks = kh * JPW + k2;
             uint32_t pa[4];
-            ldmatrix_x4(pa, sc + (rg * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * sp + kb * AT_BN + ks * 16 +
-                                (lane >> 4) * 8);
+            ldmatrix_x4_at(pa, p_at + (kb * AT_BN + ks * 16) * 2);
 #pragma unroll
             for(int jp = 0; jp < 4; ++jp)
             {
                 uint32_t vf[4];
-                ldmatrix_x4_trans(vf, tile_ptr(skv[buf], ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, 2 * jp + (lane >> 4)));
+                ldmatrix_x4_trans_at(vf, tile + ks * 2048 + v_off[jp]);
                 mma_16816(o[2 * jp], pa, vf[0], vf[1]);
                 mma_16816(o[2 * jp + 1], pa, vf[2], vf[3]);
             }
         }
-        __syncthreads();
     }
+    __syncthreads();
     // the key shares are added in a fixed order: the partial sums of shares 1 .. KS-1 go through
     // shared memory (tiles and scores are free now; (KS - 1) BMC x 64 floats = 16 or 24 KB from the start)
     float* red = reinterpret_cast<float*>(at_smem);
@@ -881,28 +971,36 @@ extern "C" int mgx_cuda_attention(const mgx_attention_desc* d, const void* q, co
         const int rows    = narrow ? 32 : AT_BM;
         const dim3 cgrid(static_cast<unsigned>((d->seq + rows - 1) / rows), grid.y, grid.z);
         const int bytes = (AT_BM * AT_D + 2 * AT_BN * AT_D + rows * sp) * 2 + 2 * AT_BM * 4;
-        // opted in once per instantiation, to the size its longest sequence needs
-        auto launch = [&](auto kernel, int max_seq) {
-            const int max_bytes = (AT_BM * AT_D + 2 * AT_BN * AT_D + AT_BM * (max_seq + 8)) * 2 + 2 * AT_BM * 4;
-            const int rc        = ensure_smem_optin(reinterpret_cast<const void*>(kernel), max_bytes);
+        auto launch = [&](auto kernel) {
+            const int rc = ensure_smem_optin(reinterpret_cast<const void*>(kernel), bytes);
             if(rc != MGX_OK)
                 return rc;
             kernel<<<cgrid, ATC_THREADS, bytes, stream>>>(p, sp);
             return static_cast<int>(cudaGetLastError());
         };
-        if(narrow)
+        switch(static_cast<int>(ceil_div(d->seq, AT_BN)))
         {
-            if(d->seq <= 384)
-                return launch(attention_f16_chain_kernel<6, 2>, 384);
-            if(d->seq <= 512)
-                return launch(attention_f16_chain_kernel<8, 2>, 512);
-            return launch(attention_f16_chain_kernel<AT_CHAIN_MAX_SEQ / 64, 2>, AT_CHAIN_MAX_SEQ);
+#define MGX_ATTENTION(NV) \
+    case NV: return narrow ? launch(attention_f16_chain_kernel<NV, 2>) : launch(attention_f16_chain_kernel<NV, 4>);
+            MGX_ATTENTION(1)
+            MGX_ATTENTION(2)
+            MGX_ATTENTION(3)
+            MGX_ATTENTION(4)
+            MGX_ATTENTION(5)
+            MGX_ATTENTION(6)
+            MGX_ATTENTION(7)
+            MGX_ATTENTION(8)
+            MGX_ATTENTION(9)
+            MGX_ATTENTION(10)
+            MGX_ATTENTION(11)
+            MGX_ATTENTION(12)
+            MGX_ATTENTION(13)
+            MGX_ATTENTION(14)
+            MGX_ATTENTION(15)
+            MGX_ATTENTION(16)
+#undef MGX_ATTENTION
         }
-        if(d->seq <= 384)
-            return launch(attention_f16_chain_kernel<6, 4>, 384);
-        if(d->seq <= 512)
-            return launch(attention_f16_chain_kernel<8, 4>, 512);
-        return launch(attention_f16_chain_kernel<AT_CHAIN_MAX_SEQ / 64, 4>, AT_CHAIN_MAX_SEQ);
+        return MGX_E_UNSUPPORTED;
     }
     else
         attention_f16_kernel<<<grid, 128, 0, stream>>>(p);

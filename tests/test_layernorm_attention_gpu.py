@@ -62,6 +62,20 @@ def test_layernorm_only_quantised_output_and_no_affine(cuda_device):
 @pytest.mark.parametrize("batch,seq,heads", [(1, 384, 12), (2, 200, 4), (3, 64, 2), (1, 77, 1), (8, 384, 12),
                                              (1, 1024, 2), (1, 1100, 2)])
 def test_attention_matches_chain(cuda_device, batch, seq, heads):
+    check_attention(cuda_device, batch, seq, heads)
+
+
+@pytest.mark.parametrize("batch", [2, 80])  # 32 and 64 query rows to a block
+@pytest.mark.parametrize("tiles", range(1, 17))
+def test_attention_at_the_edges_of_key_tiles(cuda_device, batch, tiles):
+    """A kernel of its own for every number of 64-key tiles: one key in the last one, an even and an odd number,
+    and a full one."""
+    for seq in (64 * tiles - 63, 64 * tiles - 31, 64 * tiles):
+        if batch == 2 or tiles <= 3 or seq % 64 == 33:
+            check_attention(cuda_device, batch, seq, 2 if batch == 2 else 1)
+
+
+def check_attention(cuda_device, batch, seq, heads):
     import torch
     from amdmigraphx_b200 import capi
     rng = np.random.default_rng(batch * 1000 + seq)
