@@ -3,27 +3,31 @@
 //   D[m,n] = sum_k a[m,k] * (q[n,k] - zp[n,k/group]) * s[n,k/group]
 //
 // as an fp16 x fp16 -> fp32 GEMM whose A operand is dequantised on the fly: the packed weights
-// of 128 output columns x 128 k arrive by TMA, eight warps (two threads per weight row) turn them
+// of 128 output columns x 128 k arrive by TMA, sixteen warps (four threads per weight row) turn them
 // into fp16 values (q - zp) * s and write them straight into TENSOR MEMORY, and the MMAs read
 // their A operand from there; the B operand is the caller's fp16 activation matrix, fetched by
 // TMA as it lies in memory.  The dequantised weights never exist in shared or global memory
 // (the reference materialises them: src/onnx/parse_matmulnbits.cpp:85-158 IR on the ref target).
 //
-// CTA tile = 128 output columns x 128 activation rows: all of K, persistent over tiles, or, where
-// tiles are few, a share of K and one tile.
+// CTA tile = 128 output columns x up to 192 activation rows, a multiple of 16 chosen by the launch: all of K,
+// persistent over tiles, or, where tiles are few, a share of K and one tile.
 // The tensor core cuts its running sum at every step, which pulls a long one towards zero.  So a sum
 // runs over no more than half of K: the two halves of a tile have an accumulator each and are added in
-// the epilogue, and a third one lets the next tile begin meanwhile.  Mean relative error against 64-bit
+// the epilogue, and with tiles of up to 128 rows a third one lets the next tile begin meanwhile.  Mean relative error against 64-bit
 // sums, weights and activations of one sign, with one accumulator a tile and with two: K 4096 -2.3e-5 /
-// -1.1e-5, 11008 -5.8e-5 / -2.9e-5, 28672 -1.6e-4 / -8.1e-5.  Time of the same two, 512 rows: 12288 x 4096
-// 58.6 / 59.0 us, 4096 x 11008 57.0 / 53.3, 22016 x 4096 103.4 / 103.3; 1000 rows 12288 x 4096 119.1 / 117.1.
-// CTA = 576 threads:
+// -1.1e-5, 11008 -5.8e-5 / -2.9e-5, 28672 -1.6e-4 / -8.1e-5.
+// CTA = 832 threads:
 //   warp 0       TMA producer: per 128-k group 8 KB of packed weights and 2 x 16 KB of activations
-//   warps 2..5, 10..13  dequantise (nibbles -> fp16 pairs with byte permutes, one subtract and
-//                one multiply per pair) -> tcgen05.st
 //   warp 1       MMA issuer
-//   warps 6..9, 14..17  epilogue, half of a tile's activation rows each: tcgen05.ld, add, convert,
+//   warps 2..17  dequantise (nibbles -> fp16 pairs: a byte permute, a mask, one multiply-add and one multiply per
+//                pair) -> tcgen05.st.  Two sets of eight take groups in turn, so that a group's chain from the landed
+//                bytes to the MMA has the time of two groups' MMAs
+//   warps 18..25 epilogue, half of a tile's activation rows each: tcgen05.ld, add, convert,
 //                store (consecutive lanes = consecutive n)
+// 512 rows, tiles of 128 (us), with one set of eight warps (19 instructions a word and a wait before them) and so:
+// 12288 x 4096 56.3 / 47.9, 22016 x 4096 92.0 / 82.1, 4096 x 11008 48.3 / 42.9.  What bounds it: issue slots (3200
+// instructions a group, a third of them the conversion) and the operands' stream from L2, which alone takes 34 us of
+// the first.
 // Only plain TMA loads; every wait is bounded.
 #include "common.cuh"
 #include "ptx.cuh"
@@ -34,18 +38,18 @@
 namespace mgx {
 
 constexpr int PF_ROWS    = 128; // output columns (weight rows) per tile = UMMA M
-constexpr int PF_TOKENS  = 128; // activation rows per tile = UMMA N
+constexpr int PF_MAX_TOKENS = 192; // activation rows per tile = UMMA N, at most
 constexpr int PF_GROUP_K = 128;
-constexpr int PF_STAGES  = 5;
+constexpr int PF_MAX_STAGES = 8;
 constexpr int PF_W_BYTES = PF_ROWS * PF_GROUP_K / 2;      // 8192
-constexpr int PF_A_ATOM  = PF_TOKENS * 128;               // 16384: 128 rows x 64 fp16
-constexpr int PF_STAGE   = PF_W_BYTES + 2 * PF_A_ATOM;    // 40960
 constexpr int PF_TSTAGES = 2;                             // A operand buffers in tensor memory (four: no faster)
-constexpr int PF_ACCS    = 3;                             // accumulators there
-constexpr int PF_A_COL0  = PF_ACCS * PF_TOKENS;
+constexpr int PF_MAX_ACCS = 3;                            // accumulators there
+constexpr int PF_A_COL0  = 384;                           // behind three of 128 columns or two of 192
 constexpr int PF_A_COLS  = PF_GROUP_K / 2;                // 64 columns per group
-constexpr int PF_SMEM    = PF_STAGES * PF_STAGE + 512 + 1024;
-constexpr int PF_THREADS = 576;
+constexpr int PF_SMEM    = 226 * 1024;
+constexpr int PF_DEQUANT = 16; // warps that dequantise
+constexpr int PF_EPI0    = 2 + PF_DEQUANT; // first epilogue warp
+constexpr int PF_THREADS = 32 * (PF_EPI0 + 8);
 constexpr int PF_EPI     = 256; // threads of the epilogue
 constexpr int PF_MAX_SPLIT = 8; // CTAs of a cluster
 
@@ -58,7 +62,12 @@ struct pf_params
     int group, groups_per_row, zp_const;
     int tiles_m, num_tiles;
     int split; // CTAs of a cluster that share a tile's K; then every CTA has one tile
+    int tokens, stages, accs; // activation rows of a tile; stages of the ring; accumulators
 };
+
+// Bytes of half a group's activations (64 k: 128 bytes a row) and of a stage of the ring.
+__host__ __device__ constexpr int pf_atom(int tokens) { return tokens * 128; }
+__host__ __device__ constexpr int pf_stage(int tokens) { return PF_W_BYTES + 2 * pf_atom(tokens); }
 
 // SPLIT: a cluster shares a tile's K
 template <bool SPLIT>
@@ -70,14 +79,15 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw_addr = smem_u32(smem_raw);
     uint8_t* smem           = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
-    uint8_t* bar_base       = smem + PF_STAGES * PF_STAGE;
+    const int TOKENS = p.tokens, STAGES = p.stages, ACCS = p.accs, ATOM = pf_atom(TOKENS), STAGE = pf_stage(TOKENS);
+    uint8_t* bar_base       = smem + STAGES * STAGE;
     uint64_t* full_bar      = reinterpret_cast<uint64_t*>(bar_base);
-    uint64_t* empty_bar     = full_bar + PF_STAGES;  // weights read (256) + MMAs retired (1)
-    uint64_t* unp_bar       = empty_bar + PF_STAGES; // A operand in tensor memory
+    uint64_t* empty_bar     = full_bar + PF_MAX_STAGES;  // weights read (a warp each) + MMAs retired (1)
+    uint64_t* unp_bar       = empty_bar + PF_MAX_STAGES; // A operand in tensor memory
     uint64_t* tfree_bar     = unp_bar + PF_TSTAGES;  // MMAs that read it retired
     uint64_t* accf_bar      = tfree_bar + PF_TSTAGES; // accumulator ready
-    uint64_t* acce_bar      = accf_bar + PF_ACCS;     // accumulator drained
-    uint64_t* peer_bar      = acce_bar + PF_ACCS;          // the cluster's partial results are in place
+    uint64_t* acce_bar      = accf_bar + PF_MAX_ACCS;     // accumulator drained
+    uint64_t* peer_bar      = acce_bar + PF_MAX_ACCS;          // the cluster's partial results are in place
     uint32_t* tmem_slot     = reinterpret_cast<uint32_t*>(peer_bar + 1);
     volatile uint32_t* abort_flag = tmem_slot + 1;
     float* part             = reinterpret_cast<float*>(smem); // [activation row][column], after the main loop
@@ -88,17 +98,17 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
     grid_launch_dependents();
     if(threadIdx.x == 0)
     {
-        for(int s = 0; s < PF_STAGES; ++s)
+        for(int s = 0; s < STAGES; ++s)
         {
             mbar_init(&full_bar[s], 1);
-            mbar_init(&empty_bar[s], 256 + 1);
+            mbar_init(&empty_bar[s], PF_DEQUANT / 2 + 1);
         }
         for(int s = 0; s < PF_TSTAGES; ++s)
         {
-            mbar_init(&unp_bar[s], 256);
+            mbar_init(&unp_bar[s], PF_DEQUANT / 2);
             mbar_init(&tfree_bar[s], 1);
         }
-        for(int b = 0; b < PF_ACCS; ++b)
+        for(int b = 0; b < ACCS; ++b)
         {
             mbar_init(&accf_bar[b], 1);
             mbar_init(&acce_bar[b], PF_EPI / 32);
@@ -142,7 +152,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
         for(int t = first; ok and t < p.num_tiles; t += step)
         {
             const int n0 = (t / p.tiles_m) * PF_ROWS;
-            const int m0 = (t % p.tiles_m) * PF_TOKENS;
+            const int m0 = (t % p.tiles_m) * TOKENS;
             for(int g = g_lo; g < g_hi; ++g)
             {
                 if(not mbar_wait_warp(&empty_bar[s], ph, abort_flag, 2))
@@ -152,13 +162,13 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
                 }
                 if(elect_one())
                 {
-                    uint8_t* st = smem + s * PF_STAGE;
-                    mbar_expect_tx(&full_bar[s], PF_STAGE);
+                    uint8_t* st = smem + s * STAGE;
+                    mbar_expect_tx(&full_bar[s], STAGE);
                     tma_load_2d(st, &tmap_w, &full_bar[s], g * (PF_GROUP_K / 2), n0);
                     tma_load_2d(st + PF_W_BYTES, &tmap_a, &full_bar[s], g * PF_GROUP_K, m0);
-                    tma_load_2d(st + PF_W_BYTES + PF_A_ATOM, &tmap_a, &full_bar[s], g * PF_GROUP_K + 64, m0);
+                    tma_load_2d(st + PF_W_BYTES + ATOM, &tmap_a, &full_bar[s], g * PF_GROUP_K + 64, m0);
                 }
-                if(++s == PF_STAGES)
+                if(++s == static_cast<uint32_t>(STAGES))
                     s = 0, ph ^= 1u;
             }
         }
@@ -167,9 +177,9 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
     {
         // ---------------------------------------------------- MMA issuer
         // D f32 += A f16 (weights, tensor memory) * B f16 (activation rows, K-major shared
-        // memory); M = 128, N = 128, K = 16 per instruction.  Three accumulators take turns over the
-        // segments, so that the epilogue of a tile overlaps the main loop of the next.
-        constexpr uint32_t idesc = make_idesc(1u, 0u, 0u, PF_ROWS, PF_TOKENS);
+        // memory); M = 128, N = the tile's rows, K = 16 per instruction.  The accumulators take turns over the
+        // segments: with three the epilogue of a tile overlaps the main loop of the next.
+        const uint32_t idesc = make_idesc(1u, 0u, 0u, PF_ROWS, static_cast<uint32_t>(TOKENS));
         const uint64_t bdesc0    = make_smem_desc_sw128(smem_u32(smem + PF_W_BYTES));
         uint32_t s = 0, ts = 0, tp = 0, buf = 0, bp = 1;
         bool ok    = true;
@@ -179,7 +189,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
                 const int g0 = g, g1 = g0 < g_mid ? g_mid : g_hi;
                 ok = mbar_wait_warp(&acce_bar[buf], bp, abort_flag, 4);
                 tc_fence_after_sync();
-                const uint32_t d_tmem = tmem_base + buf * PF_TOKENS;
+                const uint32_t d_tmem = tmem_base + buf * TOKENS;
                 for(; ok and g < g1; ++g)
                 {
                     // implies that the stage's TMA requests have landed
@@ -189,112 +199,107 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
                     tc_fence_after_sync();
                     if(elect_one())
                     {
-                        const uint64_t bdesc  = bdesc0 + static_cast<uint64_t>((s * PF_STAGE) >> 4);
+                        const uint64_t bdesc  = bdesc0 + static_cast<uint64_t>((s * STAGE) >> 4);
                         const uint32_t a_tmem = tmem_base + PF_A_COL0 + ts * PF_A_COLS;
 #pragma unroll
                         for(int k = 0; k < 8; ++k) // (64 k per 128-byte atom)
                             mma_f16_tmem_a(d_tmem, a_tmem + k * 8,
-                                           bdesc + static_cast<uint64_t>(((k >> 2) * PF_A_ATOM + (k & 3) * 32) >> 4), idesc,
+                                           bdesc + static_cast<uint64_t>(((k >> 2) * ATOM + (k & 3) * 32) >> 4), idesc,
                                            (g != g0 or k != 0) ? 1u : 0u);
                         tc_commit(&tfree_bar[ts]);
                         tc_commit(&empty_bar[s]);
                         if(g == g1 - 1)
                             tc_commit(&accf_bar[buf]);
                     }
-                    if(++s == PF_STAGES)
+                    if(++s == static_cast<uint32_t>(STAGES))
                         s = 0;
                     if(++ts == PF_TSTAGES)
                         ts = 0, tp ^= 1u;
                 }
-                if(++buf == PF_ACCS)
+                if(++buf == static_cast<uint32_t>(ACCS))
                     buf = 0, bp ^= 1u;
             }
     }
-    else if(warp < 6 or (warp >= 10 and warp < 14))
+    else if(warp < PF_EPI0)
     {
         // ---------------------------------------------------- dequantise: nibbles -> fp16
-        // Two threads per weight row (warps 2..5 take the first 64 k of a group, warps 10..13 the
-        // second): 32 packed bytes (64-byte swizzle: a quarter warp's 16-byte reads fall in eight
-        // different bank groups) -> 32 words of two fp16 each, in k order, to this row's lane of
-        // tensor memory.
+        // Two sets of eight warps take groups in turn, each with a place of its own in tensor memory.  In a set two
+        // threads per weight row, 64 k each: 32 packed bytes (64-byte swizzle: a quarter warp's 16-byte reads fall in
+        // eight different bank groups) -> 32 words of two fp16 each, in k order, to this row's lane of tensor memory.
+        const uint32_t set       = (warp - 2) >> 3;
+        const int half           = ((warp - 2) >> 2) & 1;
         const int row            = (warp & 3) * 32 + lane;
-        const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
+        const uint32_t a_tmem    = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + PF_A_COL0 + set * PF_A_COLS + half * 32;
         const int sw             = (row >> 1) & 3;
-        uint32_t it              = 0;
-        bool ok                  = true;
+        const uint8_t* const pk0 = smem + row * 64 + (((half * 2) ^ sw) << 4);
+        const uint8_t* const pk1 = smem + row * 64 + (((half * 2 + 1) ^ sw) << 4);
+        // A packed byte holds k (low nibble) and k + 1: as 0x6400 | q and 0x6400 | q << 4 they are the halves
+        // 1024 + q and 1024 + 16 q.  times (1, 1/16) less (1024 + zp, 64 + zp) is q - zp, exact in fp16; one
+        // rounding in the multiply with the scale
+        const __half2 unit = __halves2half2(__float2half_rn(1.0f), __float2half_rn(0.0625f));
+        auto less_zp       = [](int z) { return __halves2half2(__int2half_rn(-1024 - z), __int2half_rn(-64 - z)); };
+        __half2 zz2        = less_zp(p.zp_const);
+        uint32_t s = 0, ph = 0, turn = 0, tp = 1;
+        bool ok = true;
         for(int t = first; ok and t < p.num_tiles; t += step)
         {
             const int n  = min((t / p.tiles_m) * PF_ROWS + row, static_cast<int>(p.N) - 1);
             const unsigned short* srow =
                 reinterpret_cast<const unsigned short*>(p.scales) + static_cast<int64_t>(n) * p.groups_per_row;
             const uint8_t* zrow = p.zp == nullptr ? nullptr : p.zp + static_cast<int64_t>(n) * p.groups_per_row;
-            // scale and zero point of the next group are fetched one group ahead
-            unsigned short s_next = __ldg(srow + (g_lo >> rshift));
-            int z_next            = zrow == nullptr ? p.zp_const : static_cast<int>(__ldg(zrow + (g_lo >> rshift)));
-            for(int g = g_lo; g < g_hi; ++g, ++it)
+            // scale and zero point of this set's next group are fetched one ahead
+            int ahead             = min(g_lo + static_cast<int>(turn ^ set), g_hi - 1) >> rshift;
+            unsigned short s_next = __ldg(srow + ahead);
+            uint8_t z_next        = zrow == nullptr ? 0 : __ldg(zrow + ahead);
+#pragma unroll 1
+            for(int g = g_lo; g < g_hi; ++g, turn ^= 1u)
             {
-                const uint32_t s  = it % PF_STAGES;
-                const uint32_t ph = (it / PF_STAGES) & 1u;
-                const uint32_t ts = it % PF_TSTAGES;
-                const uint32_t tp = (it / PF_TSTAGES) & 1u;
-                const unsigned short s_cur = s_next;
-                const int z_cur            = z_next;
-                if(g + 1 < g_hi)
+                if(turn == set)
                 {
-                    const int gi = (g + 1) >> rshift;
-                    s_next       = __ldg(srow + gi);
-                    z_next       = zrow == nullptr ? p.zp_const : static_cast<int>(__ldg(zrow + gi));
-                }
-                // the tensor-memory stores below are warp-wide: leave only as a whole warp
-                if(not __all_sync(0xffffffffu, mbar_wait_bounded(&full_bar[s], ph, abort_flag, 1)) or
-                   not __all_sync(0xffffffffu, mbar_wait_bounded(&tfree_bar[ts], tp ^ 1u, abort_flag, 8)))
-                {
-                    ok = false;
-                    break;
-                }
-                tc_fence_after_sync();
-                // (1024 + q) - (1024 + zp) is exact in fp16; one rounding in the multiply
-                const uint32_t zz = 0x64006400u + static_cast<uint32_t>(z_cur) * 0x00010001u;
-                const uint32_t ss = static_cast<uint32_t>(s_cur) * 0x00010001u;
-                const __half2 zz2 = *reinterpret_cast<const __half2*>(&zz);
-                const __half2 ss2 = *reinterpret_cast<const __half2*>(&ss);
-                const uint8_t* pk = smem + s * PF_STAGE + row * 64;
-                const int half = warp >= 10 ? 1 : 0;
-                {
+                    const unsigned short s_cur = s_next;
+                    if(zrow != nullptr)
+                        zz2 = less_zp(z_next);
+                    ahead  = min(g + 2, g_hi - 1) >> rshift;
+                    s_next = __ldg(srow + ahead);
+                    if(zrow != nullptr)
+                        z_next = __ldg(zrow + ahead);
+                    // the tensor-memory stores below are warp-wide: leave only as a whole warp
+                    ok = mbar_wait_warp(&full_bar[s], ph, abort_flag, 1);
+                    if(not ok)
+                        break;
+                    const uint4 w0 = *reinterpret_cast<const uint4*>(pk0 + s * STAGE);
+                    const uint4 w1 = *reinterpret_cast<const uint4*>(pk1 + s * STAGE);
+                    __syncwarp();
+                    if(lane == 0)
+                        mbar_arrive(&empty_bar[s]); // the packed block is in registers
+                    const uint32_t ww[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+                    const uint32_t ss    = static_cast<uint32_t>(s_cur) * 0x00010001u;
+                    const __half2 ss2    = *reinterpret_cast<const __half2*>(&ss);
                     uint32_t u[32];
 #pragma unroll
-                    for(int c = 0; c < 2; ++c)
-                    {
-                        const uint4 w4 =
-                            *reinterpret_cast<const uint4*>(pk + (((half * 2 + c) ^ sw) << 4));
-                        const uint32_t ww[4] = {w4.x, w4.y, w4.z, w4.w};
+                    for(int i = 0; i < 8; ++i)
 #pragma unroll
-                        for(int i = 0; i < 4; ++i)
+                        for(int j = 0; j < 4; ++j)
                         {
-                            const uint32_t lo = ww[i] & 0x0F0F0F0Fu;        // k 0 2 4 6
-                            const uint32_t hi = (ww[i] >> 4) & 0x0F0F0F0Fu; // k 1 3 5 7
-                            const uint32_t t01 = __byte_perm(lo, hi, 0x5140); // k 0 1 2 3
-                            const uint32_t t23 = __byte_perm(lo, hi, 0x7362); // k 4 5 6 7
-                            uint32_t h[4];
-                            h[0] = __byte_perm(t01, 0x64646464u, 0x4140);
-                            h[1] = __byte_perm(t01, 0x64646464u, 0x4342);
-                            h[2] = __byte_perm(t23, 0x64646464u, 0x4140);
-                            h[3] = __byte_perm(t23, 0x64646464u, 0x4342);
-#pragma unroll
-                            for(int j = 0; j < 4; ++j)
-                            {
-                                const __half2 x = __hmul2(
-                                    __hsub2(*reinterpret_cast<const __half2*>(&h[j]), zz2), ss2);
-                                u[(c * 4 + i) * 4 + j] = *reinterpret_cast<const uint32_t*>(&x);
-                            }
+                            const uint32_t h = __byte_perm(ww[i], 0x64646464u, 0x4040u + j * 0x0101u) & 0xFFF0FF0Fu;
+                            const __half2 x  = __hmul2(__hfma2(*reinterpret_cast<const __half2*>(&h), unit, zz2), ss2);
+                            u[4 * i + j]     = *reinterpret_cast<const uint32_t*>(&x);
                         }
-                    }
-                    tmem_st_32x32b_x32(tmem_base + lane_addr + PF_A_COL0 + ts * PF_A_COLS + half * 32, u);
+                    // (the place is waited for last: the MMAs that free it run during all of the above)
+                    ok = mbar_wait_warp(&tfree_bar[set], tp, abort_flag, 8);
+                    if(not ok)
+                        break;
+                    tp ^= 1u;
+                    tc_fence_after_sync();
+                    tmem_st_32x32b_x32(a_tmem, u);
+                    tmem_st_wait();
+                    tc_fence_before_sync();
+                    __syncwarp();
+                    if(lane == 0)
+                        mbar_arrive(&unp_bar[set]);
                 }
-                mbar_arrive(&empty_bar[s]); // the packed block is in registers
-                tmem_st_wait();
-                tc_fence_before_sync();
-                mbar_arrive(&unp_bar[ts]);
+                if(++s == static_cast<uint32_t>(STAGES))
+                    s = 0, ph ^= 1u;
             }
         }
     }
@@ -302,36 +307,40 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
     {
         // ---------------------------------------------------- epilogue
         const int quarter = warp & 3;
-        const int c0      = warp >= 14 ? PF_TOKENS / 2 : 0; // this warp's activation rows of the tile
+        // this warp's activation rows of the tile, 16 at a time
+        const int chunks = TOKENS / 16, lower = (chunks + 1) / 2;
+        const int c0 = warp >= PF_EPI0 + 4 ? lower * 16 : 0, mine = warp >= PF_EPI0 + 4 ? chunks - lower : lower;
         const int segs    = g_mid < g_hi ? 2 : 1;
         uint32_t buf = 0, bp = 0;
         for(int t = first; t < p.num_tiles; t += step)
         {
             const int64_t n  = static_cast<int64_t>(t / p.tiles_m) * PF_ROWS + quarter * 32 + lane;
-            const int64_t m0 = static_cast<int64_t>(t % p.tiles_m) * PF_TOKENS;
+            const int64_t m0 = static_cast<int64_t>(t % p.tiles_m) * TOKENS;
             const uint32_t buf0 = buf;
             bool ok = true;
             for(int i = 0; ok and i < segs; ++i)
             {
                 ok = mbar_wait_warp(&accf_bar[buf], bp, abort_flag, 3);
-                if(++buf == PF_ACCS)
+                if(++buf == static_cast<uint32_t>(ACCS))
                     buf = 0, bp ^= 1u;
             }
             // (in a cluster a wait that gave up goes on without waiting: the barriers below need every thread)
             if(not SPLIT and not ok)
                 break;
-            const uint32_t buf1 = buf0 + 1 == PF_ACCS ? 0 : buf0 + 1;
+            const uint32_t buf1 = buf0 + 1 == static_cast<uint32_t>(ACCS) ? 0 : buf0 + 1;
             tc_fence_after_sync();
             const uint32_t tbase = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + c0;
+            __half* dst    = p.D + (m0 + c0) * p.ldd + n;
+            const int rows = static_cast<int>(min(p.M - m0 - c0, static_cast<int64_t>(mine * 16))); // of this warp's that exist
 #pragma unroll 1
-            for(int c = 0; c < PF_TOKENS / 32; ++c)
+            for(int c = 0; c < mine; ++c)
             {
                 uint32_t acc[16];
-                tmem_ld_32x32b_x16(tbase + buf0 * PF_TOKENS + c * 16, acc);
+                tmem_ld_32x32b_x16(tbase + buf0 * TOKENS + c * 16, acc);
                 if(not SPLIT and segs == 2)
                 {
                     uint32_t acc1[16];
-                    tmem_ld_32x32b_x16(tbase + buf1 * PF_TOKENS + c * 16, acc1);
+                    tmem_ld_32x32b_x16(tbase + buf1 * TOKENS + c * 16, acc1);
                     tmem_ld_wait();
 #pragma unroll
                     for(int j = 0; j < 16; ++j)
@@ -349,12 +358,9 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
                 else if(n < p.N)
                 {
 #pragma unroll
-                    for(int j = 0; j < 16; ++j)
-                    {
-                        const int64_t m = m0 + c0 + c * 16 + j;
-                        if(m < p.M)
-                            p.D[m * p.ldd + n] = __float2half_rn(__uint_as_float(acc[j]));
-                    }
+                    for(int j = 0; j < 16; ++j, dst += p.ldd)
+                        if(c * 16 + j < rows)
+                            *dst = __float2half_rn(__uint_as_float(acc[j]));
                 }
             }
             tc_fence_before_sync();
@@ -369,7 +375,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
             {
                 // CTA r adds up the r-th share of the tile's columns, four at a time
                 asm volatile("bar.sync 1, %0;" ::"n"(PF_EPI) : "memory");
-                const int et = static_cast<int>(threadIdx.x) - (warp >= 14 ? 320 : 192);
+                const int et = static_cast<int>(threadIdx.x) - 32 * PF_EPI0;
                 if(et < p.split)
                     cluster_arrive(peer_bar, et);
                 if(ok and __all_sync(0xffffffffu, mbar_wait_cluster_bounded(peer_bar, 0u, abort_flag, 6)))
@@ -377,7 +383,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
                     const int share = PF_ROWS / p.split, per = share / 4;
                     const int col   = rank * share + et % per * 4;
                     const int64_t n4 = static_cast<int64_t>(t / p.tiles_m) * PF_ROWS + col;
-                    for(int m = et / per; m < PF_TOKENS and m0 + m < p.M; m += PF_EPI / per)
+                    for(int m = et / per; m < TOKENS and m0 + m < p.M; m += PF_EPI / per)
                     {
                         float v[PF_MAX_SPLIT][4], sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
@@ -483,6 +489,41 @@ int max_clusters(int split)
     return n;
 }
 
+// The rows of a tile and the split of its K with the smallest estimated time, in cycles: waves of tiles, each its
+// groups at the slowest of the MMAs, the operands' stream from L2 (62 bytes per cycle) and the dequantising warps, then
+// what the epilogue keeps to itself.  (512 rows, 12288 x 4096: 384 tiles of 128 rows are two and a half waves, 47.9 us,
+// 288 of 176 rows two, 41.8; 4096 x 11008: 128 tiles of 128 rows 43.1, 96 of 176 48.9.  1000 rows, 12288 x 4096: 92.6 and
+// 81.6.)
+// K is shared by a cluster where tiles are few, each CTA at least four groups, and only where all the clusters run at
+// once, as one left over costs a second wave (24 tokens, 4096 x 11008, 32 tiles: 44 us in one CTA each, 17 us; 16
+// tiles of K 4096, eight CTAs each 17.6 us, four 10.7; 36 tiles of K 11008, four 36.3, two 29.3).
+void pf_plan(const mgx_w4_desc& d, pf_params& p)
+{
+    const int64_t tiles_n = ceil_div(d.N, PF_ROWS), groups = d.K / PF_GROUP_K, sms = device_sm_count();
+    double best = 0.0;
+    for(int64_t tiles_m = ceil_div(d.M, PF_MAX_TOKENS); tiles_m <= ceil_div(d.M, 64); ++tiles_m)
+    {
+        const int tokens    = static_cast<int>(ceil_div(ceil_div(d.M, tiles_m), 16) * 16);
+        const int64_t tiles = tiles_n * tiles_m;
+        int split           = 1;
+        for(int s = 2; s <= PF_MAX_SPLIT and groups >= 4 * s and tiles <= max_clusters(s); s *= 2)
+            split = s;
+        const double group = std::max({4.0 * tokens, pf_stage(tokens) / 62.0, 560.0}) + 100.0;
+        const double waves = split > 1 ? 1.0 : static_cast<double>(ceil_div(tiles, sms));
+        const double alone = 12.0 * tokens; // the last tile's epilogue, and every one's with two accumulators
+        const double cost  = waves * ceil_div(groups, split) * group + (tokens > 128 ? waves : 1.0) * alone + (split > 1 ? 2500.0 : 0.0);
+        if(best != 0.0 and cost >= best)
+            continue;
+        best        = cost;
+        p.tokens    = tokens;
+        p.tiles_m   = static_cast<int>(tiles_m);
+        p.num_tiles = static_cast<int>(tiles);
+        p.split     = split;
+    }
+    p.accs   = p.tokens <= 128 ? 3 : 2;
+    p.stages = static_cast<int>(std::min<int64_t>(PF_MAX_STAGES, (PF_SMEM - 1536) / pf_stage(p.tokens)));
+}
+
 } // namespace
 
 bool w4a16_prefill_applicable(const mgx_w4_desc& d, const void* A, const void* Bp)
@@ -491,7 +532,7 @@ bool w4a16_prefill_applicable(const mgx_w4_desc& d, const void* A, const void* B
     return d.M > 16 and d.K % PF_GROUP_K == 0 and d.group % PF_GROUP_K == 0 and
            (ratio & (ratio - 1)) == 0 and d.act == MGX_ACT_NONE and d.lda % 8 == 0 and
            ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(Bp)) & 15u) == 0 and
-           ceil_div(d.N, PF_ROWS) * ceil_div(d.M, PF_TOKENS) < (int64_t{1} << 30) and
+           ceil_div(d.N, PF_ROWS) * ceil_div(d.M, 64) < (int64_t{1} << 30) and
            d.N * (d.K / d.group) < (int64_t{1} << 40);
 }
 
@@ -502,11 +543,6 @@ int w4a16_prefill_launch(const mgx_w4_desc& d, const void* A, const void* Bp, co
     int rc = encode_rows(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, Bp, static_cast<uint64_t>(d.K / 2),
                          static_cast<uint64_t>(d.N), static_cast<uint64_t>(d.K / 2), PF_GROUP_K / 2,
                          PF_ROWS, CU_TENSOR_MAP_SWIZZLE_64B);
-    if(rc != MGX_OK)
-        return rc;
-    rc = encode_rows(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT16, A, static_cast<uint64_t>(d.K),
-                     static_cast<uint64_t>(d.M), static_cast<uint64_t>(d.lda) * 2, 64, PF_TOKENS,
-                     CU_TENSOR_MAP_SWIZZLE_128B);
     if(rc != MGX_OK)
         return rc;
     pf_params p{};
@@ -520,22 +556,17 @@ int w4a16_prefill_launch(const mgx_w4_desc& d, const void* A, const void* Bp, co
     p.group          = d.group;
     p.groups_per_row = static_cast<int>(d.K / d.group);
     p.zp_const       = d.zp_const;
-    p.tiles_m        = static_cast<int>(ceil_div(d.M, PF_TOKENS));
-    p.num_tiles      = static_cast<int>(ceil_div(d.N, PF_ROWS)) * p.tiles_m;
-    // Few tiles leave SMs idle: a cluster shares a tile's K, each CTA at least four groups, and adds its
-    // partial results through distributed shared memory (24 tokens, 4096 x 11008, 32 tiles: 44 us in one
-    // CTA each, 17 us).  Only where all the clusters run at once, as one left over costs a second wave: 16 tiles
-    // of K 4096, eight CTAs each 17.6 us, four 10.7; 36 tiles of K 11008, four 36.3, two 29.3.
     rc = ensure_smem_optin(reinterpret_cast<const void*>(w4a16_prefill_kernel<true>), PF_SMEM);
+    if(rc == MGX_OK)
+        rc = ensure_smem_optin(reinterpret_cast<const void*>(w4a16_prefill_kernel<false>), PF_SMEM);
     if(rc != MGX_OK)
         return rc;
-    p.split = 1;
-    for(int s = 2; s <= PF_MAX_SPLIT and d.K / PF_GROUP_K >= 4 * s and p.num_tiles <= max_clusters(s); s *= 2)
-        p.split = s;
+    pf_plan(d, p);
+    rc = encode_rows(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT16, A, static_cast<uint64_t>(d.K), static_cast<uint64_t>(d.M),
+                     static_cast<uint64_t>(d.lda) * 2, 64, static_cast<uint32_t>(p.tokens), CU_TENSOR_MAP_SWIZZLE_128B);
+    if(rc != MGX_OK)
+        return rc;
     auto* kernel = p.split > 1 ? w4a16_prefill_kernel<true> : w4a16_prefill_kernel<false>;
-    rc           = ensure_smem_optin(reinterpret_cast<const void*>(kernel), PF_SMEM);
-    if(rc != MGX_OK)
-        return rc;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
     configure(cfg, attr, p.split > 1 ? p.num_tiles : std::min(p.num_tiles, device_sm_count()), p.split, stream);
