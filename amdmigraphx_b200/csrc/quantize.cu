@@ -562,6 +562,47 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// The same with 16-byte accesses: 64 x 64 elements a block, rows of 72 in shared memory so that the eight elements a
+// thread gathers down a column lie in different banks from its neighbours'.  A prompt's values (32 x 512 x 128, 8 MB
+// moved) 5.6 us an element at a time, 4.6 so.
+__global__ void __launch_bounds__(256)
+    transpose_16bit_vec_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ dst, int64_t rows, int64_t cols,
+                               int64_t ld_dst)
+{
+    __shared__ __align__(16) uint16_t tile[64][72];
+    grid_dependency_wait();
+    const uint16_t* s = src + blockIdx.z * rows * cols;
+    uint16_t* d       = dst + blockIdx.z * cols * ld_dst;
+    const int64_t r0 = static_cast<int64_t>(blockIdx.y) * 64, c0 = static_cast<int64_t>(blockIdx.x) * 64;
+#pragma unroll
+    for(int i = 0; i < 2; ++i)
+    {
+        const int u = threadIdx.x + i * 256, rr = u >> 3, cc = (u & 7) * 8;
+        if(r0 + rr < rows and c0 + cc < cols)
+            *reinterpret_cast<uint4*>(&tile[rr][cc]) = *reinterpret_cast<const uint4*>(s + (r0 + rr) * cols + c0 + cc);
+    }
+    grid_launch_dependents();
+    __syncthreads();
+#pragma unroll
+    for(int i = 0; i < 2; ++i)
+    {
+        // column of src = row of dst; eight of its elements
+        const int u = threadIdx.x + i * 256, cc = u >> 3, rr = (u & 7) * 8;
+        if(c0 + cc >= cols or r0 + rr >= rows)
+            continue;
+        uint32_t w[4];
+#pragma unroll
+        for(int e = 0; e < 4; ++e)
+            w[e] = tile[rr + 2 * e][cc] | static_cast<uint32_t>(tile[rr + 2 * e + 1][cc]) << 16;
+        uint16_t* at = d + (c0 + cc) * ld_dst + r0 + rr;
+        if(r0 + rr + 8 <= rows)
+            *reinterpret_cast<uint4*>(at) = make_uint4(w[0], w[1], w[2], w[3]);
+        else
+            for(int e = 0; r0 + rr + e < rows; ++e)
+                at[e] = static_cast<uint16_t>(w[e >> 1] >> (16 * (e & 1)));
+    }
+}
+
 int transpose_16bit_ld(const void* src, void* dst, int64_t rows, int64_t cols, int64_t batch,
                        int64_t ld_dst, cudaStream_t stream)
 {
@@ -570,6 +611,12 @@ int transpose_16bit_ld(const void* src, void* dst, int64_t rows, int64_t cols, i
     const int64_t gx = ceil_div(cols, 32), gy = ceil_div(rows, 32);
     if(gy > 65535 or batch > 65535)
         return MGX_E_TOO_LARGE;
+    if(cols % 8 == 0 and ld_dst % 8 == 0 and (reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) % 16 == 0)
+        return launch_dependent(transpose_16bit_vec_kernel,
+                                dim3(static_cast<unsigned>(ceil_div(cols, 64)), static_cast<unsigned>(ceil_div(rows, 64)),
+                                     static_cast<unsigned>(batch)),
+                                dim3(256), 0, stream, static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), rows, cols,
+                                ld_dst);
     dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy), static_cast<unsigned>(batch));
     transpose_16bit_kernel<<<grid, 256, 0, stream>>>(static_cast<const uint16_t*>(src),
                                                      static_cast<uint16_t*>(dst), rows, cols, ld_dst);

@@ -54,6 +54,13 @@ def test_f16_dot_kn_batched(cuda_device, batch, M, N, K):
         _check(got[i], a[i], b[i], True)
 
 
+@pytest.mark.parametrize("batch,M,N,K", [(1, 24, 8, 8), (2, 40, 72, 100), (1, 33, 136, 65), (3, 16, 64, 63), (2, 64, 128, 512)])
+def test_f16_dot_kn_operand_in_vectors(cuda_device, batch, M, N, K):
+    """Rows of the [K,N] operand are whole 16-byte vectors: it is re-laid out 64 x 64 at a time, with ragged last
+    vectors along K."""
+    test_f16_dot_kn_batched(cuda_device, batch, M, N, K)
+
+
 def test_f16_dot_bias_relu_residual(cuda_device):
     import torch
     from amdmigraphx_b200 import capi

@@ -183,3 +183,25 @@ def test_masked_scale_form(cuda_device, lens, op, swap, scalar_inputs):
     got = capi.pointwise(ins, prog, lens).cpu().numpy()
     ref = _numpy_program(nps, prog).astype(np.float16)
     np.testing.assert_array_equal(got.view(np.uint16), ref.view(np.uint16))
+
+
+@pytest.mark.parametrize("dtype", ["float16", "float32"])
+@pytest.mark.parametrize("shape,order", [
+    ((3, 40, 8), (1, 0, 2)), ((32, 65, 128), (1, 0, 2)), ((2, 3, 5, 16), (2, 0, 1, 3)), ((1, 7, 24), (1, 0, 2)),
+    ((4, 6, 12), (1, 0, 2)),   # rows that are not whole vectors: the register machine
+    ((4, 6, 16), (2, 0, 1)),   # rows that are not contiguous: the register machine
+])
+def test_identity_of_a_transposed_view(cuda_device, dtype, shape, order):
+    """The copy kernel and the register machine give the input's bits, infinities and zeros of both signs among
+    them."""
+    import torch
+    from amdmigraphx_b200 import capi
+    g = torch.Generator(device=cuda_device)
+    g.manual_seed(sum(shape))
+    x = torch.randn(shape, generator=g, device=cuda_device).to(getattr(torch, dtype))
+    x.view(-1)[:4] = torch.tensor([float("inf"), -float("inf"), 0.0, -0.0], dtype=x.dtype)
+    view = x.permute(order)
+    code = capi.F16 if dtype == "float16" else capi.F32
+    out = capi.pointwise([view], [("identity", code, (0,), 0.0)], tuple(view.shape))
+    bits = torch.int16 if dtype == "float16" else torch.int32
+    assert torch.equal(out.view(bits), view.contiguous().view(bits))
