@@ -466,6 +466,61 @@ __device__ __forceinline__ void tmem_ld_wait()
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// ------------------------------------------------------------- pairs of CTAs (cta_group::2)
+// The two CTAs of a cluster of two work on one accumulator of 256 rows: CTA r holds rows 128 r .. 128 r + 127 of D in
+// its own tensor memory, and in its own shared memory the same rows of A and the r-th half of the rows of B, at the
+// same offsets as the other.  CTA 0 issues.  Allocation and release take a warp of each.
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_slot, uint32_t ncols)
+{
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_slot)), "r"(ncols)
+                 : "memory");
+}
+
+__device__ __forceinline__ void tmem_relinquish_pair()
+{
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols)
+{
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+
+// Into this CTA's shared memory, completion on CTA 0's barrier (the one at the same place as `bar`).
+__device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int32_t c0, int32_t c1,
+                                                 int32_t c2)
+{
+    asm volatile("{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %2, 0;\n\t"
+                 "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2"
+                 " [%0], [%1, {%3, %4, %5}], [r];\n\t}" ::"r"(smem_u32(smem_dst)),
+                 "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
+                 : "memory");
+}
+
+// Arrive on the barrier of both CTAs when all tcgen05.mma issued so far by this thread finish.
+__device__ __forceinline__ void tc_commit_pair(uint64_t* bar)
+{
+    const uint16_t both = 3;
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+                     smem_u32(bar)),
+                 "h"(both)
+                 : "memory");
+}
+
+#define MGX_MMA_PAIR(NAME, KIND)                                                                                       \
+    __device__ __forceinline__ void NAME(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,            \
+                                         uint32_t accumulate)                                                          \
+    {                                                                                                                  \
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"                                               \
+                     "tcgen05.mma.cta_group::2.kind::" KIND " [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),                \
+                     "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)                                             \
+                     : "memory");                                                                                      \
+    }
+MGX_MMA_PAIR(mma_i8_pair, "i8")
+MGX_MMA_PAIR(mma_f8_pair, "f8f6f4")
+MGX_MMA_PAIR(mma_f16_pair, "f16")
+#undef MGX_MMA_PAIR
+
 // ------------------------------------------------------------- descriptors
 // Shared-memory matrix descriptor for a K-major operand tile stored as rows of
 // 128 bytes with the 128-byte swizzle (what a TMA box {128 B, rows} with

@@ -417,3 +417,61 @@ def test_ragged_rows_take_the_vector_epilogue(cuda_device, M):
     np.testing.assert_array_equal(out[0, :M].cpu().numpy().view(np.uint16), ref.view(np.uint16))
     np.testing.assert_array_equal(q[0, :M].cpu().numpy(), O.quantizelinear(ref, np.array([0.03125], dtype=np.float16)))
     assert (out[0, M:] == 7.0).all() and (q[0, M:] == 9).all()
+
+
+# (on 148 SMs: 256 x 224, 192, 224, 192, 192 with more than eight rows of tiles, 128, 256)
+PAIRS = [(257, 8190, 8208), (700, 4000, 2000), (1000, 8180, 8192), (2300, 4100, 4112), (2500, 1030, 6160), (250, 8200, 8192),
+         (2040, 4090, 4096)]
+
+
+@pytest.mark.parametrize("M,N,K", PAIRS)
+def test_tiles_of_two_ctas_int8_bit_exact(cuda_device, M, N, K):
+    """Ragged last tiles in M, N and K, several tiles per pair; int32 exact (8-bit products, summed in int64 here)."""
+    import torch
+    from amdmigraphx_b200 import capi
+    rng = np.random.default_rng(M + N + K)
+    a, w = _rand_i8(rng, (M, K)), _rand_i8(rng, (N, K))
+    out = torch.full((1, M + 8, N), 7, dtype=torch.int32, device=cuda_device)
+    capi.qgemm(_t(a, cuda_device), _t(w, cuda_device), b_layout=capi.B_NK, out=out[:, :M])
+    # 2^14 x 8208 < 2^53: fp64 products of int8 values are exact
+    ref = torch.from_numpy(a).to(cuda_device).double() @ torch.from_numpy(w).to(cuda_device).double().T
+    assert torch.equal(out[0, :M].double(), ref) and (out[0, M:] == 7).all()
+    assert capi.device_status() == 0
+
+
+@pytest.mark.parametrize("kind", ["fp8", "f16"])
+@pytest.mark.parametrize("M,N,K", PAIRS)
+def test_tiles_of_two_ctas_fp(cuda_device, M, N, K, kind):
+    """Against fp64: the accumulators are fp32 sums of exact products, |error| <= K 2^-24 |a| |b| in any order; the
+    bound here is 4e-6 of that product, the half result one step of a half more."""
+    import torch
+    from amdmigraphx_b200 import capi
+    g = torch.Generator(device=cuda_device).manual_seed(M + N + K)
+    qt = torch.float8_e4m3fn if kind == "fp8" else torch.float16
+    a = torch.randn(M, K, generator=g, device=cuda_device).to(qt)
+    w = torch.randn(N, K, generator=g, device=cuda_device).to(qt)
+    bias = torch.randn(N, generator=g, device=cuda_device)
+    got = capi.qgemm(a, w, b_layout=capi.B_NK, bias=bias, act="relu", out_dtype=torch.float16).double()
+    ref = torch.relu(a.double() @ w.double().T + bias.double())
+    mag = a.double().abs() @ w.double().abs().T + bias.double().abs()
+    assert ((got - ref).abs() <= 4e-6 * mag + ref.abs() * 2.0 ** -10 + 2.0 ** -24).all()
+
+
+def test_tiles_of_two_ctas_residual_and_quantised_result(cuda_device):
+    import torch
+    from amdmigraphx_b200 import capi
+    M, N, K = 700, 4000, 2000
+    rng = np.random.default_rng(5)
+    a, w = _rand_i8(rng, (M, K)), _rand_i8(rng, (N, K))
+    scale = rng.uniform(1e-6, 1e-5, size=N).astype(np.float32)
+    bias = rng.normal(0, 0.5, size=N).astype(np.float32)
+    res = rng.normal(size=(M, N)).astype(np.float16)
+    out = torch.full((1, M + 8, N), 7.0, dtype=torch.float16, device=cuda_device)
+    q = torch.full((1, M + 8, N), 9, dtype=torch.int8, device=cuda_device)
+    capi.qgemm(_t(a, cuda_device), _t(w, cuda_device), b_layout=capi.B_NK, scale=_t(scale, cuda_device),
+               bias=_t(bias, cuda_device), residual=_t(res, cuda_device), out=out[:, :M], q_out=q[:, :M], q_scale=0.03125)
+    acc = (torch.from_numpy(a).to(cuda_device).double() @ torch.from_numpy(w).to(cuda_device).double().T).cpu().numpy()
+    ref = O.qlinear_epilogue(acc.astype(np.int32), scale[None, :], bias, None, res, np.float16)
+    np.testing.assert_array_equal(out[0, :M].cpu().numpy().view(np.uint16), ref.view(np.uint16))
+    np.testing.assert_array_equal(q[0, :M].cpu().numpy(), O.quantizelinear(ref, np.array([0.03125], dtype=np.float16)))
+    assert (out[0, M:] == 7.0).all() and (q[0, M:] == 9).all()
