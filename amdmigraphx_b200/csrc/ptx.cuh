@@ -188,6 +188,17 @@ __device__ __forceinline__ uint32_t cluster_load(const void* p, uint32_t rank)
     return v;
 }
 
+__device__ __forceinline__ uint4 cluster_load_uint4(const void* p, uint32_t rank)
+{
+    uint4 v;
+    asm volatile("{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %4, %5;\n\t"
+                 "ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [r];\n\t}"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "r"(smem_u32(p)), "r"(rank)
+                 : "memory");
+    return v;
+}
+
 __device__ __forceinline__ void cluster_load4(const float* p, uint32_t rank, float (&v)[4])
 {
     asm volatile("{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %4, %5;\n\t"

@@ -16,16 +16,21 @@ namespace mgx {
 // at most 4 % off the fastest, 0.5 % on average.  Pairs against the best tile of one CTA, int8 / fp8: 8192^3 405 -> 328
 // us, 1000 x 8192 x 8192 57.5 / 61.4 -> 49.5 / 54.4 (224: 148 pairs' tiles, two full waves), 6144 x 1024 x 4096 27.1 ->
 // 22.3, 700 x 4000 x 2000 18.8 -> 14.5; but 1024^3 5.7 -> 7.9 and 3072 x 3072 x 768 16.6 -> 18.3, where K is short.
+// Tiles of 128 x 64 that are so few that clusters of 2, 4 or 8 CTAs with a share of K each all run at once: a k-block costs
+// the same, the launch of clusters and the exchange of their sums 2740 (1.2 us) + 25 per CTA + 230 (S - 2) more, fitted
+// to 24 shapes.  Against the best without: 100 x 1000 x 4096 9.3 -> 6.6 us, 20 x 2048 x 8192 14.4 -> 9.2, 200 x 768 x 3072
+// 7.2 -> 6.5, 512 x 1024 x 4096 9.3 -> 8.5; but 128 x 2048 x 2048 6.1 -> 6.6 by four, 256 x 1024 x 1024 4.4 -> 5.2 by two.
 struct tile_choice
 {
     bool pair;
     int bn;
+    int split = 1; // CTAs that share a tile's K
 };
 
 static tile_choice pick_tile(const mgx_qgemm_desc& d)
 {
     // tuning knob: MGX_CUDA_QGEMM_BN = 64 | 128 | 256 forces tiles of one CTA of that width, 1128 | 1192 | 1224 | 1256
-    // tiles of a pair
+    // tiles of a pair, 2002 | 2004 | 2008 a shared K
     static const int forced = [] {
         const char* e = std::getenv("MGX_CUDA_QGEMM_BN");
         return e != nullptr ? std::atoi(e) : 0;
@@ -46,6 +51,18 @@ static tile_choice pick_tile(const mgx_qgemm_desc& d)
         const double cost   = waves * std::max(main, epi) + 0.25 * std::min(main, epi) + (c.pair ? 2858.0 : 0.0);
         if(best_cost == 0.0 or cost < best_cost)
             best_cost = cost, best = c;
+    }
+    for(int split : {2, 4, 8})
+    {
+        if(split > kb)
+            break;
+        if(forced == 2000 + split)
+            return {false, 64, split};
+        const int64_t tiles = ceil_div(d.M, 128) * ceil_div(d.N, 64) * d.batch;
+        const double cost   = static_cast<double>(ceil_div(static_cast<int64_t>(kb), split)) * 2.44 * 192 + 3478.0 +
+                            25.0 * static_cast<double>(tiles * split) + 230.0 * (split - 2);
+        if(forced == 0 and tiles <= qgemm_split_clusters(split) and cost < best_cost)
+            best_cost = cost, best = {false, 64, split};
     }
     return best;
 }
@@ -171,6 +188,8 @@ extern "C" int mgx_cuda_qgemm_ex(const mgx_qgemm_desc* d, const void* A, const v
         return qgemv_launch(*d, A, Bk, D, scale, bias, ldb, stream);
     const qgemm_operands o{A, Bk, D, scale, bias, residual, ldb, stride_b};
     const tile_choice tile = pick_tile(*d);
+    if(tile.split > 1)
+        return qgemm_split_launch(tile.split, *d, o, qo, stream);
     const auto launch = d->ab_type == MGX_I8 ? (tile.pair ? qgemm_pair_i8_launch : qgemm_i8_launch)
                         : f16                ? (tile.pair ? qgemm_pair_f16_launch : qgemm_f16_launch)
                                              : (tile.pair ? qgemm_pair_f8_launch : qgemm_f8_launch);
@@ -180,7 +199,7 @@ extern "C" int mgx_cuda_qgemm_ex(const mgx_qgemm_desc* d, const void* A, const v
 int mgx::qgemm_status(unsigned int* out)
 {
     *out = 0;
-    for(auto f : {qgemm_i8_status, qgemm_f8_status, qgemm_f16_status, qgemm_pair_i8_status, qgemm_pair_f8_status, qgemm_pair_f16_status})
+    for(auto f : {qgemm_i8_status, qgemm_f8_status, qgemm_f16_status, qgemm_pair_i8_status, qgemm_pair_f8_status, qgemm_pair_f16_status, qgemm_split_status})
     {
         unsigned int v = 0;
         const int rc   = f(&v);

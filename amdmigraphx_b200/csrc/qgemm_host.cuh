@@ -42,4 +42,9 @@ int qgemm_pair_i8_status(unsigned int* out);
 int qgemm_pair_f8_status(unsigned int* out);
 int qgemm_pair_f16_status(unsigned int* out);
 
+// tiles of 128 x 64 whose K is shared by the split (2, 4 or 8) CTAs of a cluster, and how many such clusters run at once
+int qgemm_split_launch(int split, const mgx_qgemm_desc& d, const qgemm_operands& o, const qout_args& qo, cudaStream_t stream);
+int qgemm_split_clusters(int split);
+int qgemm_split_status(unsigned int* out);
+
 } // namespace mgx

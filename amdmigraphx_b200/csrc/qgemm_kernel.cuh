@@ -20,6 +20,11 @@
 // of the tile's columns of B, and holds its 128 rows of D; the MMAs, issued by the first CTA, read B from both.
 // What a k-block takes out of L2 per SM falls from 128 + BN rows to 128 + BN / 2, which is what bounds a tile of one
 // CTA: 8192^3 int8 405 -> 328 us (3.35 POPS, tensor pipe at the clock the power allows), 1000 x 8192 x 8192 fp8 61 -> 54.
+//
+// SPLIT: the S CTAs of a cluster work on one tile of 128 x 64, each on its share of K; the grid is as many clusters as
+// there are tiles.  The partial accumulators are exchanged through shared memory where the stages were, every warp
+// adding (in the order of the ranks) and finishing 32 / S rows of 16 columns.  For few tiles and long K:
+// one CTA walks a k-block in 0.2 us, 100 x 1000 x 4096 fp8 9.3 -> 6.6 us.
 #pragma once
 #include "common.cuh"
 #include "ptx.cuh"
@@ -46,6 +51,7 @@ struct qgemm_params
     const float* bias;
     const void* residual;
     int tiles_m, tiles_n, group_m;
+    int split; // CTAs that share a tile's K: 2, 4 or 8 (SPLIT)
     int64_t num_tiles;
     int num_kb;
     int scale_mode;
@@ -131,6 +137,7 @@ struct epi_ctx
 {
     const qgemm_params* p;
     uint8_t* box;      // this warp's 32 x 64-byte staging area (16-byte pieces XOR-swizzled by row)
+    int rows;          // of it in use
     int lane;
     int64_t row0;      // global row of staging row 0
     int64_t batch_off; // b * stride_d
@@ -158,7 +165,7 @@ __device__ __forceinline__ void epi_store_chunk(const epi_ctx& e, int64_t col, f
         const int64_t row = e.row0 + r;
         const uint4 w =
             *reinterpret_cast<const uint4*>(e.box + r * 64 + ((pc ^ ((r >> 1) & 3)) * 16));
-        if(row >= p.M or c4 >= p.N)
+        if(r >= e.rows or row >= p.M or c4 >= p.N)
             continue;
         const uint32_t wv[4] = {w.x, w.y, w.z, w.w};
         OutT* dst = static_cast<OutT*>(p.D) + e.batch_off + row * p.ldd + c4;
@@ -392,7 +399,7 @@ __device__ __forceinline__ void epi_store_chunk_fast(const epi_ctx& e, int64_t c
     const uint32_t hmask = p.hmask;
     const uint8_t* box = e.box + rsub * 64;
     // (rows beyond M: only in the last row of tiles; one comparison per four values)
-    const int rows = static_cast<int>(min(p.M - e.row0, int64_t{32}));
+    const int rows = static_cast<int>(min(p.M - e.row0, static_cast<int64_t>(e.rows)));
 #pragma unroll 2
     for(int it = 0; it < 4; ++it)
     {
@@ -525,8 +532,8 @@ __device__ __forceinline__ void epi_store_chunk_fast(const epi_ctx& e, int64_t c
 // tile's columns.  Per 16-column chunk: tcgen05.ld (one row per thread) -> swizzled shared
 // memory -> read back with 4 lanes per 64-byte row segment -> dequantizelinear / bias /
 // activation / residual -> coalesced global stores.
-template <int BN, bool IS_INT, class OutT, int ACT, int MODE, bool PAIR>
-__device__ __forceinline__ void epilogue_role(const qgemm_params& p, uint8_t* epi_base,
+template <int BN, bool IS_INT, class OutT, int ACT, int MODE, bool PAIR, bool SPLIT>
+__device__ __forceinline__ void epilogue_role(const qgemm_params& p, uint8_t* epi_base, uint8_t* part, uint64_t* peer_bar,
                                               uint64_t* accf_bar, uint64_t* acce_bar,
                                               volatile uint32_t* abort_flag, uint32_t tmem_base,
                                               int warp, int lane, int64_t first_tile,
@@ -537,14 +544,16 @@ __device__ __forceinline__ void epilogue_role(const qgemm_params& p, uint8_t* ep
     const int slice   = ew >> 2;
     // this warp's chunks of the tile's columns: a quarter of them, or as near to it as whole chunks allow
     constexpr int CHUNKS = BN / EPI_COLS;
-    const int ch_lo      = CHUNKS % 4 == 0 ? slice * (CHUNKS / 4) : slice * CHUNKS / 4;
-    const int nchunk     = CHUNKS % 4 == 0 ? CHUNKS / 4 : (slice + 1) * CHUNKS / 4 - ch_lo;
+    // (the first case apart: one more register, and the int8 kernel of 128 columns spills)
+    const int col_lo     = CHUNKS % 4 == 0 ? slice * (BN / 4) : slice * CHUNKS / 4 * EPI_COLS;
+    const int nchunk     = CHUNKS % 4 == 0 ? CHUNKS / 4 : (slice + 1) * CHUNKS / 4 - slice * CHUNKS / 4;
     constexpr int ROWS   = PAIR ? 2 * BM : BM; // of a tile
     const int row_cta    = PAIR ? static_cast<int>(blockIdx.x & 1) * BM : 0;
     epi_ctx e;
     e.p    = &p;
     e.box  = epi_base + ew * (32 * EPI_COLS * 4);
     e.lane = lane;
+    e.rows = 32;
     uint8_t* my_row    = e.box + lane * 64;
     const int my_swz   = (lane >> 1) & 3;
     const bool per_col = p.scale_mode == MGX_SCALE_PER_COL;
@@ -557,8 +566,17 @@ __device__ __forceinline__ void epilogue_role(const qgemm_params& p, uint8_t* ep
         int m_blk, n_blk;
         tile_place<PAIR>(p, r, m_blk, n_blk);
         const uint32_t buf = lt & 1u;
-        const int64_t col0 = static_cast<int64_t>(n_blk) * BN + ch_lo * EPI_COLS;
-        e.row0      = static_cast<int64_t>(m_blk) * ROWS + row_cta + quarter * 32;
+        int64_t col0 = static_cast<int64_t>(n_blk) * BN + col_lo;
+        e.row0       = static_cast<int64_t>(m_blk) * ROWS + row_cta + quarter * 32;
+        // SPLIT: unit u = 4 x chunk + quarter of the tile is finished by CTA u / units, S warps to a unit
+        const int units = SPLIT ? EPI_WARPS / p.split : 1;
+        const int unit  = SPLIT ? static_cast<int>(blockIdx.x) % p.split * units + ew / p.split : 0;
+        if constexpr(SPLIT)
+        {
+            e.rows = 32 / p.split;
+            col0   = static_cast<int64_t>(n_blk) * BN + (unit >> 2) * EPI_COLS;
+            e.row0 = static_cast<int64_t>(m_blk) * BM + (unit & 3) * 32 + ew % p.split * e.rows;
+        }
         e.batch_off = b * p.stride_d;
         e.batch_off_q = b * p.stride_q;
 
@@ -623,6 +641,63 @@ __device__ __forceinline__ void epilogue_role(const qgemm_params& p, uint8_t* ep
             break;
         tc_fence_after_sync();
 
+        if constexpr(SPLIT)
+        {
+            static_assert(BN == 4 * EPI_COLS and not PAIR, "one chunk per warp");
+            uint32_t acc[EPI_COLS];
+            __syncwarp();
+            tmem_ld_32x32b_x16(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + slice * EPI_COLS, acc);
+            tmem_ld_wait();
+            // (the accumulator being complete, the MMAs have read all that was in the stages)
+            const int mine = slice * 4 + quarter;
+            uint8_t* row   = part + mine * 2048 + lane * 64;
+#pragma unroll
+            for(int q = 0; q < 4; ++q)
+                *reinterpret_cast<uint4*>(row + ((q ^ my_swz) * 16)) =
+                    make_uint4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
+            __syncwarp();
+            if(lane == 0)
+                cluster_arrive(peer_bar, mine / units);
+            // units x S = 16 arrivals: all this CTA's units are in place in all CTAs
+            if(not __all_sync(0xffffffffu, mbar_wait_cluster_bounded(peer_bar, 0, abort_flag, 6)))
+                break;
+            for(int i = lane; i < e.rows * 4; i += 32)
+            {
+                const int r = i >> 2, pc = i & 3, from = ew % p.split * e.rows + r;
+                const uint8_t* src = part + unit * 2048 + from * 64 + ((pc ^ ((from >> 1) & 3)) * 16);
+                uint4 v[8];
+#pragma unroll
+                for(int k = 0; k < 8; ++k)
+                    if(k < p.split)
+                        v[k] = cluster_load_uint4(src, k);
+                uint4 sum = v[0];
+#pragma unroll
+                for(int k = 1; k < 8; ++k)
+                    if(k < p.split)
+                    {
+                        if constexpr(IS_INT)
+                            sum.x += v[k].x, sum.y += v[k].y, sum.z += v[k].z, sum.w += v[k].w;
+                        else
+                        {
+                            sum.x = __float_as_uint(__uint_as_float(sum.x) + __uint_as_float(v[k].x));
+                            sum.y = __float_as_uint(__uint_as_float(sum.y) + __uint_as_float(v[k].y));
+                            sum.z = __float_as_uint(__uint_as_float(sum.z) + __uint_as_float(v[k].z));
+                            sum.w = __float_as_uint(__uint_as_float(sum.w) + __uint_as_float(v[k].w));
+                        }
+                    }
+                *reinterpret_cast<uint4*>(e.box + r * 64 + ((pc ^ ((r >> 1) & 3)) * 16)) = sum;
+            }
+            __syncwarp();
+            if(col0 < p.N)
+            {
+                if constexpr(MODE != 0 and not std::is_same<OutT, int32_t>::value)
+                    epi_store_chunk_fast<IS_INT, OutT, ACT, MODE>(e, col0, sc_next, bi_next);
+                else
+                    epi_store_chunk<IS_INT, OutT, ACT>(e, col0, sc_next, bi_next);
+            }
+            break; // one tile per cluster
+        }
+
 #pragma unroll 1
         for(int ch = 0; ch < nchunk; ++ch)
         {
@@ -636,7 +711,7 @@ __device__ __forceinline__ void epilogue_role(const qgemm_params& p, uint8_t* ep
             uint32_t acc[EPI_COLS];
             __syncwarp(); // tcgen05.ld is warp-collective; also orders reuse of the box
             const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
-                                   buf * ACC_COLS<BN> + (ch_lo + ch) * EPI_COLS;
+                                   buf * ACC_COLS<BN> + col_lo + ch * EPI_COLS;
             tmem_ld_32x32b_x16(taddr, acc);
             tmem_ld_wait();
             if(col < p.N)
@@ -669,7 +744,7 @@ __device__ __forceinline__ void epilogue_role(const qgemm_params& p, uint8_t* ep
 // OutT: int32_t (raw accumulator), float or __half.
 // F16: the operands are fp16 (kind::f16, 64 elements of K per 128-byte stage row); the byte
 // layout of the pipeline is the one of the 8-bit kinds.
-template <int BN, bool IS_INT, class OutT, bool F16, bool PAIR>
+template <int BN, bool IS_INT, class OutT, bool F16, bool PAIR, bool SPLIT>
 __global__ void __launch_bounds__(NTHREADS, 1)
     qgemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
                  const __grid_constant__ CUtensorMap tmap_b,
@@ -686,7 +761,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     uint64_t* empty_bar = full_bar + S::stages;
     uint64_t* accf_bar  = empty_bar + S::stages; // [2] accumulator ready
     uint64_t* acce_bar  = accf_bar + 2;          // [2] accumulator drained
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acce_bar + 2);
+    uint64_t* peer_bar  = acce_bar + 2;          // SPLIT: the cluster's partial sums are in place
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(peer_bar + 1);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
     const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
@@ -709,6 +785,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             mbar_init(&accf_bar[b], 1);
             mbar_init(&acce_bar[b], PAIR ? 2 * EPI_WARPS : EPI_WARPS); // one arrival per epilogue warp
         }
+        mbar_init(peer_bar, EPI_WARPS);
         *abort_flag = 0;
         fence_barrier_init();
         prefetch_tensormap(&tmap_a);
@@ -728,18 +805,22 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         }
     }
     tc_fence_before_sync();
-    if constexpr(PAIR)
+    if constexpr(PAIR or SPLIT)
     {
         __syncwarp();
-        cluster_barrier(); // both CTAs' barriers exist and their tensor memory is allocated
+        cluster_barrier(); // all its CTAs' barriers exist, a pair's tensor memory is allocated
     }
     else
         __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
 
-    const int64_t first_tile = PAIR ? blockIdx.x >> 1 : blockIdx.x;
-    const int64_t tile_step  = PAIR ? gridDim.x >> 1 : gridDim.x;
+    const int64_t first_tile = SPLIT ? blockIdx.x / p.split : PAIR ? blockIdx.x >> 1 : blockIdx.x;
+    const int64_t tile_step  = SPLIT ? p.num_tiles : PAIR ? gridDim.x >> 1 : gridDim.x;
+    // this CTA's blocks of K
+    const int share = SPLIT ? static_cast<int>(blockIdx.x) % p.split : 0;
+    const int kb_lo = SPLIT ? p.num_kb * share / p.split : 0;
+    const int kb_hi = SPLIT ? p.num_kb * (share + 1) / p.split : p.num_kb;
     const int64_t tiles_mn   = static_cast<int64_t>(p.tiles_m) * p.tiles_n;
 
     if(warp == 0)
@@ -756,7 +837,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             const int r     = static_cast<int>(t % tiles_mn);
             int m_blk, n_blk;
             tile_place<PAIR>(p, r, m_blk, n_blk);
-            for(int kb = 0; kb < p.num_kb; ++kb)
+            for(int kb = kb_lo; kb < kb_hi; ++kb)
             {
                 if(not mbar_wait_warp(&empty_bar[s], ph, abort_flag, 2))
                 {
@@ -813,7 +894,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 break;
             tc_fence_after_sync();
             const uint32_t d_tmem = tmem_base + buf * ACC_COLS<BN>;
-            for(int kb = 0; kb < p.num_kb; ++kb)
+            for(int kb = kb_lo; kb < kb_hi; ++kb)
             {
                 if(not mbar_wait_warp(&full_bar[s], ph, abort_flag, 1))
                 {
@@ -831,29 +912,29 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                         // advancing K inside the 128-byte swizzle row: +32 B on the start address
                         const uint64_t koff = static_cast<uint64_t>((k * UMMA_K) >> 4);
                         if constexpr(PAIR and IS_INT)
-                            mma_i8_pair(d_tmem, adesc + koff, bdesc + koff, idesc, (kb | k) != 0);
+                            mma_i8_pair(d_tmem, adesc + koff, bdesc + koff, idesc, ((kb - kb_lo) | k) != 0);
                         else if constexpr(PAIR and F16)
-                            mma_f16_pair(d_tmem, adesc + koff, bdesc + koff, idesc, (kb | k) != 0);
+                            mma_f16_pair(d_tmem, adesc + koff, bdesc + koff, idesc, ((kb - kb_lo) | k) != 0);
                         else if constexpr(PAIR)
-                            mma_f8_pair(d_tmem, adesc + koff, bdesc + koff, idesc, (kb | k) != 0);
+                            mma_f8_pair(d_tmem, adesc + koff, bdesc + koff, idesc, ((kb - kb_lo) | k) != 0);
                         else if constexpr(IS_INT)
-                            mma_i8(d_tmem, adesc + koff, bdesc + koff, idesc, (kb | k) != 0);
+                            mma_i8(d_tmem, adesc + koff, bdesc + koff, idesc, ((kb - kb_lo) | k) != 0);
                         else if constexpr(F16)
-                            mma_f16(d_tmem, adesc + koff, bdesc + koff, idesc, (kb | k) != 0);
+                            mma_f16(d_tmem, adesc + koff, bdesc + koff, idesc, ((kb - kb_lo) | k) != 0);
                         else
-                            mma_f8(d_tmem, adesc + koff, bdesc + koff, idesc, (kb | k) != 0);
+                            mma_f8(d_tmem, adesc + koff, bdesc + koff, idesc, ((kb - kb_lo) | k) != 0);
                     }
                     // the stage is reusable once these MMAs have read it; after the last, the accumulator complete
                     if constexpr(PAIR)
                     {
                         tc_commit_pair(&empty_bar[s]);
-                        if(kb == p.num_kb - 1)
+                        if(kb == kb_hi - 1)
                             tc_commit_pair(&accf_bar[buf]);
                     }
                     else
                     {
                         tc_commit(&empty_bar[s]);
-                        if(kb == p.num_kb - 1)
+                        if(kb == kb_hi - 1)
                             tc_commit(&accf_bar[buf]);
                     }
                 }
@@ -870,8 +951,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         // the check-free variant is chosen once per launch: the tile loop a warp runs holds
         // only the store path it takes
 #define MGX_EPI_MODE(ACT, MODE)                                                                           \
-    epilogue_role<BN, IS_INT, OutT, ACT, MODE, PAIR>(p, epi_base, accf_bar, acce_bar, abort_flag, tmem_base, warp, \
-                                                     lane, first_tile, tile_step, tiles_mn)
+    epilogue_role<BN, IS_INT, OutT, ACT, MODE, PAIR, SPLIT>(p, epi_base, smem, peer_bar, accf_bar, acce_bar, abort_flag, \
+                                                            tmem_base, warp, lane, first_tile, tile_step, tiles_mn)
 // (fp16 operands have no quantised result, and only int32 accumulators a mode of their own below 2^24)
 #define MGX_EPI_IF(COND, ACT, MODE) \
     if constexpr(COND)              \
@@ -926,10 +1007,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             __nanosleep(1000);
     }
     tc_fence_before_sync();
-    if constexpr(PAIR)
+    if constexpr(PAIR or SPLIT)
     {
-        // neither CTA leaves, or frees tensor memory, while the other may still read its operands, arrive on its
-        // barriers or read its half of an accumulator
+        // no CTA leaves, or frees a pair's tensor memory, while another may still read its operands or partial sums or
+        // arrive on its barriers
         __syncwarp();
         cluster_barrier();
     }
@@ -966,10 +1047,10 @@ static int encode_operand_map(CUtensorMap* map, const void* base, int64_t k, int
     return r == CUDA_SUCCESS ? MGX_OK : MGX_E_INVALID_ARG;
 }
 
-template <int BN, bool IS_INT, class OutT, bool F16, bool PAIR>
+template <int BN, bool IS_INT, class OutT, bool F16, bool PAIR, bool SPLIT>
 static int launch_qgemm(const mgx_qgemm_desc& d, const void* A, const void* B, void* D,
                         const float* scale, const float* bias, const void* residual,
-                        int64_t ldb, int64_t stride_b, const qout_args& qo, cudaStream_t stream)
+                        int64_t ldb, int64_t stride_b, const qout_args& qo, int split, cudaStream_t stream)
 {
     using S = qgemm_smem<BN, PAIR>;
     CUtensorMap ta, tb;
@@ -1001,6 +1082,7 @@ static int launch_qgemm(const mgx_qgemm_desc& d, const void* A, const void* B, v
     p.residual   = residual;
     p.tiles_m    = static_cast<int>(ceil_div(d.M, PAIR ? 2 * BM : BM));
     p.tiles_n    = static_cast<int>((d.N + BN - 1) / BN);
+    p.split      = split;
     p.group_m    = PAIR ? (p.tiles_m < 8 ? p.tiles_m : 8) : p.tiles_m;
     p.num_tiles  = static_cast<int64_t>(p.tiles_m) * p.tiles_n * d.batch;
     p.num_kb     = static_cast<int>((d.K * ab + BK - 1) / BK);
@@ -1040,13 +1122,14 @@ static int launch_qgemm(const mgx_qgemm_desc& d, const void* A, const void* B, v
     // whatever its low bits; no zero point may shift the rounding boundary
     p.q_mask     = (qo.Dq != nullptr and qo.fp8 == 0 and qo.scale >= 0.000244140625f and
                     qo.zp == static_cast<float>(static_cast<int>(qo.zp))) ? 1 : 0;
-    auto kernel  = qgemm_kernel<BN, IS_INT, OutT, F16, PAIR>;
+    auto kernel  = qgemm_kernel<BN, IS_INT, OutT, F16, PAIR, SPLIT>;
     int rc2 = ensure_smem_optin(reinterpret_cast<const void*>(kernel), S::total);
     if(rc2 != MGX_OK)
         return rc2;
     // (every group of SMs that clusters are placed in has an even number of them)
     const int sms  = PAIR ? device_sm_count() / 2 : device_sm_count();
-    const int grid = static_cast<int>(p.num_tiles < sms ? p.num_tiles : sms) * (PAIR ? 2 : 1);
+    const int grid = SPLIT ? static_cast<int>(p.num_tiles) * split
+                           : static_cast<int>(p.num_tiles < sms ? p.num_tiles : sms) * (PAIR ? 2 : 1);
     // programmatic dependent launch: set-up (tensor-memory allocation, barriers, descriptor
     // prefetch) overlaps the tail of the previous kernel of the stream
     cudaLaunchConfig_t cfg{};
@@ -1058,27 +1141,27 @@ static int launch_qgemm(const mgx_qgemm_desc& d, const void* A, const void* B, v
     attr[0].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     attr[1].id               = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = 2;
+    attr[1].val.clusterDim.x = static_cast<unsigned>(PAIR ? 2 : split);
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs                                          = attr;
-    cfg.numAttrs                                       = PAIR ? 2 : 1;
+    cfg.numAttrs                                       = PAIR or SPLIT ? 2 : 1;
     return static_cast<int>(cudaLaunchKernelEx(&cfg, kernel, ta, tb, p));
 }
 
-template <int BN, bool IS_INT, bool F16, bool PAIR>
-static int dispatch_out(const mgx_qgemm_desc& d, const qgemm_operands& o, const qout_args& qo, cudaStream_t stream)
+template <int BN, bool IS_INT, bool F16, bool PAIR, bool SPLIT = false>
+static int dispatch_out(const mgx_qgemm_desc& d, const qgemm_operands& o, const qout_args& qo, cudaStream_t stream, int split = 1)
 {
     switch(d.out_type)
     {
     case MGX_I32:
         if constexpr(IS_INT)
-            return launch_qgemm<BN, true, int32_t, false, PAIR>(d, o.A, o.B, o.D, o.scale, o.bias, o.residual, o.ldb, o.stride_b, qo, stream);
+            return launch_qgemm<BN, true, int32_t, false, PAIR, SPLIT>(d, o.A, o.B, o.D, o.scale, o.bias, o.residual, o.ldb, o.stride_b, qo, split, stream);
         else
             return MGX_E_UNSUPPORTED;
     case MGX_F32:
-        return launch_qgemm<BN, IS_INT, float, F16, PAIR>(d, o.A, o.B, o.D, o.scale, o.bias, o.residual, o.ldb, o.stride_b, qo, stream);
+        return launch_qgemm<BN, IS_INT, float, F16, PAIR, SPLIT>(d, o.A, o.B, o.D, o.scale, o.bias, o.residual, o.ldb, o.stride_b, qo, split, stream);
     case MGX_F16:
-        return launch_qgemm<BN, IS_INT, __half, F16, PAIR>(d, o.A, o.B, o.D, o.scale, o.bias, o.residual, o.ldb, o.stride_b, qo, stream);
+        return launch_qgemm<BN, IS_INT, __half, F16, PAIR, SPLIT>(d, o.A, o.B, o.D, o.scale, o.bias, o.residual, o.ldb, o.stride_b, qo, split, stream);
     default: return MGX_E_UNSUPPORTED;
     }
 }

@@ -475,3 +475,47 @@ def test_tiles_of_two_ctas_residual_and_quantised_result(cuda_device):
     np.testing.assert_array_equal(out[0, :M].cpu().numpy().view(np.uint16), ref.view(np.uint16))
     np.testing.assert_array_equal(q[0, :M].cpu().numpy(), O.quantizelinear(ref, np.array([0.03125], dtype=np.float16)))
     assert (out[0, M:] == 7.0).all() and (q[0, M:] == 9).all()
+
+
+# (K shared by two, four and eight CTAs of a cluster on 148 SMs; ragged rows, columns and shares of K)
+SHARED_K = [(384, 768, 3072), (100, 1000, 4112), (17, 130, 8176), (129, 600, 4800), (500, 1000, 4224), (33, 17, 8992)]
+
+
+@pytest.mark.parametrize("M,N,K", SHARED_K)
+def test_shared_k_int8_bit_exact(cuda_device, M, N, K):
+    import torch
+    from amdmigraphx_b200 import capi
+    rng = np.random.default_rng(M + N + K)
+    a, w = _rand_i8(rng, (M, K)), _rand_i8(rng, (N, K))
+    ref = O.quant_dot_int8(a, w.T)
+    out = torch.full((1, M + 8, N), 7, dtype=torch.int32, device=cuda_device)
+    capi.qgemm(_t(a, cuda_device), _t(w, cuda_device), b_layout=capi.B_NK, out=out[:, :M])
+    np.testing.assert_array_equal(out[0, :M].cpu().numpy(), ref)
+    assert (out[0, M:] == 7).all()
+    scale = rng.uniform(1e-6, 1e-5, size=N).astype(np.float32)
+    bias = rng.normal(0, 0.5, size=N).astype(np.float32)
+    res = rng.normal(size=(M, N)).astype(np.float16)
+    half = torch.full((1, M + 8, N), 7.0, dtype=torch.float16, device=cuda_device)
+    capi.qgemm(_t(a, cuda_device), _t(w, cuda_device), b_layout=capi.B_NK, scale=_t(scale, cuda_device),
+               bias=_t(bias, cuda_device), residual=_t(res, cuda_device), out=half[:, :M])
+    want = O.qlinear_epilogue(ref, scale[None, :], bias, None, res, np.float16)
+    np.testing.assert_array_equal(half[0, :M].cpu().numpy().view(np.uint16), want.view(np.uint16))
+    assert (half[0, M:] == 7.0).all()
+    assert capi.device_status() == 0
+
+
+@pytest.mark.parametrize("kind", ["fp8", "f16"])
+@pytest.mark.parametrize("M,N,K", SHARED_K)
+def test_shared_k_fp(cuda_device, M, N, K, kind):
+    """fp32 partial sums added in the order of the shares: the bound of one accumulator holds for their sum."""
+    import torch
+    from amdmigraphx_b200 import capi
+    g = torch.Generator(device=cuda_device).manual_seed(M + N + K)
+    qt = torch.float8_e4m3fn if kind == "fp8" else torch.float16
+    a = torch.randn(M, K, generator=g, device=cuda_device).to(qt)
+    w = torch.randn(N, K, generator=g, device=cuda_device).to(qt)
+    bias = torch.randn(N, generator=g, device=cuda_device)
+    got = capi.qgemm(a, w, b_layout=capi.B_NK, bias=bias, out_dtype=torch.float32).double()
+    ref = a.double() @ w.double().T + bias.double()
+    mag = a.double().abs() @ w.double().abs().T + bias.double().abs()
+    assert ((got - ref).abs() <= 4e-6 * mag).all()
