@@ -10,12 +10,16 @@
 // (int32: exact; fp32: fixed order).  No partial sums, counters or second kernel in global memory: with
 // the (128-column tile, k-block) items dealt out evenly and tiles completed by the last CTA to arrive,
 // half of a small linear's time was that exchange (one row, 4096 x 4096 fp8: 10.7 us, now 7.6; 16 rows,
-// 14336 x 4096: 23.4 us, now 15.0 = 3.9 TB/s).
+// 14336 x 4096: 23.4 us, then 15.0).
 // The epilogue is the tiled GEMM's arithmetic (dequantizelinear, bias, activation, fp32 / fp16 /
 // raw int32 output; op::quant_dot + dequantizelinear.hpp:60-82 + the fused pointwise module).
 //
-// CTA = 192 threads: warp 0 TMA producer, warp 1 MMA issuer + tensor-memory owner, warps 2..5
-// epilogue.  Only plain TMA loads; every wait is bounded.
+// CTA = 192 to 576 threads: warp 0 TMA producer, warp 1 MMA issuer + tensor-memory owner, the others
+// epilogue, for every four rows one to each quarter of the columns.  The last block's epilogue is not hidden:
+// with one warp to a quarter for all rows a lane's sixteen GELUs in turn were 2 us (16 rows, fp8 with GELU,
+// 14336 x 4096 14.1 -> 12.3 us, 4096 x 4096 9.2 -> 7.9, int8 8192 x 1024 8.2 -> 5.5); with 576 threads for
+// few rows the larger block starts later (one row, 4096 x 4096 7.35 -> 7.7).  Only plain TMA loads; every wait
+// is bounded.
 #include "common.cuh"
 #include "ptx.cuh"
 #include "qgemm_math.cuh"
@@ -36,7 +40,8 @@ constexpr int GV_A_BYTES = GV_MB * GV_BK;   // 2048
 constexpr int GV_STAGE   = GV_W_BYTES + GV_A_BYTES;
 constexpr int GV_PART    = GV_MB * GV_ROWS * 4; // a block's raw accumulators: [row of A][column]
 constexpr int GV_SMEM    = GV_STAGES * GV_STAGE + 2 * GV_PART + 256 + 1024;
-constexpr int GV_THREADS = 192;
+constexpr int GV_RPW     = 4; // rows of A that an epilogue warp takes
+constexpr int GV_THREADS = 64 + GV_MB / GV_RPW * GV_ROWS; // at most
 constexpr int GV_MAX_SPLIT = 8; // CTAs of a cluster; divides GV_ROWS
 
 struct gv_params
@@ -84,7 +89,7 @@ __global__ void __launch_bounds__(GV_THREADS, 1)
         for(int b = 0; b < 2; ++b)
         {
             mbar_init(&accf_bar[b], 1);
-            mbar_init(&acce_bar[b], 4);
+            mbar_init(&acce_bar[b], (blockDim.x - 64) / 32);
         }
         mbar_init(peer_bar, p.split);
         *abort_flag = 0;
@@ -197,6 +202,8 @@ __global__ void __launch_bounds__(GV_THREADS, 1)
         // ---------------------------------------------------- epilogue
         grid_dependency_wait(); // D free to overwrite
         const int quarter = warp & 3;
+        const int row0    = (warp - 2) / 4 * GV_RPW;
+        const int epi     = static_cast<int>(blockDim.x) - 64; // threads
         const float tensor_scale = p.scale_mode == MGX_SCALE_PER_TENSOR ? __ldg(p.scale) : 1.0f;
         // raw accumulator -> output value, as in the tiled GEMM's epilogue
         auto finish = [&](uint32_t raw, float s, float b) {
@@ -256,8 +263,8 @@ __global__ void __launch_bounds__(GV_THREADS, 1)
             if(not dead and not mbar_wait_warp(&accf_bar[buf], (blk >> 1) & 1u, abort_flag, 3))
                 dead = true;
             tc_fence_after_sync();
-            uint32_t acc[GV_MB];
-            tmem_ld_32x32b_x16(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * GV_MB, acc);
+            uint32_t acc[GV_RPW];
+            tmem_ld_32x32b_x4(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * GV_MB + row0, acc);
             tmem_ld_wait();
             tc_fence_before_sync();
             __syncwarp();
@@ -268,29 +275,29 @@ __global__ void __launch_bounds__(GV_THREADS, 1)
                 if(col < cols and not dead)
                 {
 #pragma unroll
-                    for(int m = 0; m < GV_MB; ++m)
-                        if(m < p.M)
-                            store(m, n0 + col, acc[m], s, b);
+                    for(int m = 0; m < GV_RPW; ++m)
+                        if(row0 + m < p.M)
+                            store(row0 + m, n0 + col, acc[m], s, b);
                 }
                 continue;
             }
             uint32_t* mine = part + buf * (GV_MB * GV_ROWS);
 #pragma unroll
-            for(int m = 0; m < GV_MB; ++m)
-                if(m < p.M)
-                    mine[m * GV_ROWS + col] = acc[m];
+            for(int m = 0; m < GV_RPW; ++m)
+                if(row0 + m < p.M)
+                    mine[(row0 + m) * GV_ROWS + col] = acc[m];
             // CTA r finishes the r-th share of the columns.  A buffer is written again two blocks later,
             // after the exchange of the next block, which every thread reaches after it has read this one.
             const int share = GV_ROWS / p.split;
             const int c     = rank * share + et % share;
             column(n0 + c, s, b);
-            asm volatile("bar.sync 1, 128;" ::: "memory");
+            asm volatile("bar.sync 1, %0;" ::"r"(epi) : "memory");
             if(et < p.split)
                 cluster_arrive(peer_bar, et);
             if(not dead and not __all_sync(0xffffffffu, mbar_wait_cluster_bounded(peer_bar, blk & 1, abort_flag, 6)))
                 dead = true;
             if(c < cols and not dead)
-                for(int m = et / share; m < p.M; m += p.split)
+                for(int m = et / share; m < p.M; m += epi / share)
                 {
                     uint32_t tot = IS_INT ? 0u : __float_as_uint(0.0f);
 #pragma unroll
@@ -348,11 +355,11 @@ int encode_k_major(CUtensorMap* map, const void* base, uint64_t k, uint64_t rows
     return r == CUDA_SUCCESS ? MGX_OK : MGX_E_INVALID_ARG;
 }
 
-void configure(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2], int clusters, int split, cudaStream_t stream)
+void configure(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2], int clusters, int split, int threads, cudaStream_t stream)
 {
     cfg                  = cudaLaunchConfig_t{};
     cfg.gridDim          = dim3(static_cast<unsigned>(clusters * split));
-    cfg.blockDim         = dim3(GV_THREADS);
+    cfg.blockDim         = dim3(static_cast<unsigned>(threads));
     cfg.dynamicSmemBytes = GV_SMEM;
     cfg.stream           = stream;
     attr[0].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -381,7 +388,7 @@ int max_clusters(int split)
     {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[2];
-        configure(cfg, attr, device_sm_count() / split, split, nullptr);
+        configure(cfg, attr, device_sm_count() / split, split, GV_THREADS, nullptr);
         attr[0]      = attr[1];
         cfg.numAttrs = 1;
         if(cudaOccupancyMaxActiveClusters(&n, qgemv_kernel<IS_INT, OutT>, &cfg) != cudaSuccess or n < 1)
@@ -418,7 +425,7 @@ int launch_gv(const CUtensorMap& tw, const CUtensorMap& ta, gv_params p, cudaStr
     }
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
-    configure(cfg, attr, p.clusters, p.split, stream);
+    configure(cfg, attr, p.clusters, p.split, 64 + static_cast<int>(ceil_div(p.M, GV_RPW)) * GV_ROWS, stream);
     return static_cast<int>(cudaLaunchKernelEx(&cfg, kernel, tw, ta, p));
 }
 
