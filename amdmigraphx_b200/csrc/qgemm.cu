@@ -61,7 +61,7 @@ static tile_choice pick_tile(const mgx_qgemm_desc& d)
         const int64_t tiles = ceil_div(d.M, 128) * ceil_div(d.N, 64) * d.batch;
         const double cost   = static_cast<double>(ceil_div(static_cast<int64_t>(kb), split)) * 2.44 * 192 + 3478.0 +
                             25.0 * static_cast<double>(tiles * split) + 230.0 * (split - 2);
-        if(forced == 0 and tiles <= qgemm_split_clusters(split) and cost < best_cost)
+        if(forced == 0 and cost < best_cost and tiles * split <= sms and tiles <= qgemm_split_clusters(split))
             best_cost = cost, best = {false, 64, split};
     }
     return best;

@@ -13,6 +13,10 @@ int qgemm_split_launch(int split, const mgx_qgemm_desc& d, const qgemm_operands&
     return dispatch_out<64, false, false, false, true>(d, o, qo, stream, split);
 }
 
+// Stands in for the kernels in the question how many clusters fit: what limits them is the block and its shared memory,
+// the same for all, and to ask for one of them would load its code.
+__global__ void __launch_bounds__(NTHREADS, 1) split_probe_kernel() {}
+
 int qgemm_split_clusters(int split)
 {
     static std::mutex m;
@@ -25,7 +29,7 @@ int qgemm_split_clusters(int split)
     if(n == 0)
     {
         using S     = qgemm_smem<64, false>;
-        auto kernel = qgemm_kernel<64, true, float, false, false, true>; // (the same block and shared memory for every type)
+        auto kernel = split_probe_kernel;
         cudaLaunchConfig_t cfg{};
         cfg.gridDim          = dim3(static_cast<unsigned>(device_sm_count() / split * split));
         cfg.blockDim         = dim3(NTHREADS);
