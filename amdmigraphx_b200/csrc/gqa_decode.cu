@@ -437,7 +437,6 @@ __global__ void __launch_bounds__(GD_THREADS + 32, 2)
     if(*abort_flag != 0)
         for(int i = 0; i < 1000; ++i)
             __nanosleep(1000); // copies in flight land before shared memory is released
-    __syncwarp();
     if(p.split > 1)
         cluster_barrier(); // no CTA leaves while another may read its shared memory
 }

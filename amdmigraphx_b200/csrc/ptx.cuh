@@ -208,14 +208,26 @@ __device__ __forceinline__ void cluster_load4(const float* p, uint32_t rank, flo
                  : "memory");
 }
 
-__device__ __forceinline__ void cluster_barrier()
+// Barriers of whole warps (.aligned): the lanes of a warp have to execute one together, which after code that divided
+// them is only sure behind __syncwarp().
+__device__ __forceinline__ void cluster_barrier_arrive()
 {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 }
 
-// Its two halves: every thread of the cluster's CTAs passes both.
-__device__ __forceinline__ void cluster_barrier_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_barrier_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_barrier_wait()
+{
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Every thread of the cluster's CTAs passes both halves.
+__device__ __forceinline__ void cluster_barrier()
+{
+    cluster_barrier_arrive();
+    cluster_barrier_wait();
+}
 
 // ---------------------------------------------------------------- programmatic dependent launch
 // A kernel launched with cudaLaunchAttributeProgrammaticStreamSerialization may start while the

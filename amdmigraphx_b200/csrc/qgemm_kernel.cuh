@@ -806,10 +806,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     }
     tc_fence_before_sync();
     if constexpr(PAIR or SPLIT)
-    {
-        __syncwarp();
         cluster_barrier(); // all its CTAs' barriers exist, a pair's tensor memory is allocated
-    }
     else
         __syncthreads();
     tc_fence_after_sync();
@@ -1011,7 +1008,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     {
         // no CTA leaves, or frees a pair's tensor memory, while another may still read its operands or partial sums or
         // arrive on its barriers
-        __syncwarp();
         cluster_barrier();
     }
     else

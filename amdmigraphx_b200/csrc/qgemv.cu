@@ -330,10 +330,7 @@ __global__ void __launch_bounds__(GV_THREADS, 1)
         tmem_dealloc(tmem_base, 32);
     }
     if(p.split > 1)
-    {
-        __syncwarp();
         cluster_barrier(); // no CTA leaves while another may read its partial sums
-    }
 }
 
 // ------------------------------------------------------------------ host

@@ -420,10 +420,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
         tmem_dealloc(tmem_base, 512);
     }
     if constexpr(SPLIT)
-    {
-        __syncwarp();
         cluster_barrier(); // no CTA leaves while another may read its partial result
-    }
 }
 
 // ------------------------------------------------------------------ host
