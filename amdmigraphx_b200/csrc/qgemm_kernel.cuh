@@ -865,6 +865,17 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                     s = 0, ph ^= 1u;
             }
         }
+        if constexpr(PAIR)
+        {
+            // The first CTA's MMAs release the stages of both.  The last release of each is waited for here too, so that
+            // none arrives at a CTA that has left (a stage that was never filled is free).
+            for(int i = 0; ok and i < S::stages; ++i)
+            {
+                ok = mbar_wait_warp(&empty_bar[s], ph, abort_flag, 2);
+                if(++s == S::stages)
+                    s = 0, ph ^= 1u;
+            }
+        }
     }
     else if(warp == 1)
     {

@@ -18,3 +18,16 @@ def test_cluster_barriers_stand_behind_a_reconvergence(path):
     for m in re.finditer(r'asm volatile\(\s*"[^;]*barrier\.cluster\.', text):
         before = text[:m.start()].rstrip()
         assert before.endswith("__syncwarp();"), text[max(0, m.start() - 100):m.end()]
+
+
+def test_stages_released_from_another_cta_are_waited_for_at_the_end():
+    """tc_commit_pair arrives on the barriers of both CTAs of a pair.  A producer that waits for a stage only before it
+    fills it again leaves the last release of every stage unobserved, and its CTA may be gone when that arrives: behind
+    its loop over the tiles it waits for all stages once more."""
+    for path in SOURCES:
+        with open(path) as f:
+            text = f.read()
+        if "tc_commit_pair(&empty_bar" not in text:
+            continue
+        producer = text[text.index("TMA producer\n"):text.index("MMA issuer\n")]
+        assert re.search(r"if constexpr\(PAIR\)\s*\{[^{}]*for\([^{}]*S::stages[^{}]*\{[^{}]*mbar_wait_warp\(&empty_bar\[s\]", producer), path
