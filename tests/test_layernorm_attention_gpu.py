@@ -6,6 +6,7 @@ this repository's tests, rtol 2e-2 / atol 1e-2, and far tighter in practice."""
 import numpy as np
 import pytest
 
+from launched import launched
 from oracle import mgx_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -65,14 +66,22 @@ def test_attention_matches_chain(cuda_device, batch, seq, heads):
     check_attention(cuda_device, batch, seq, heads)
 
 
-@pytest.mark.parametrize("batch", [2, 80])  # 32 and 64 query rows to a block
+@pytest.mark.parametrize("groups", [2, 4])  # of 16 query rows to a block
 @pytest.mark.parametrize("tiles", range(1, 17))
-def test_attention_at_the_edges_of_key_tiles(cuda_device, batch, tiles):
-    """A kernel of its own for every number of 64-key tiles: one key in the last one, an even and an odd number,
-    and a full one."""
+def test_attention_at_the_edges_of_key_tiles(cuda_device, groups, tiles):
+    """A kernel of its own for every number of 64-key tiles and both heights of a block: one key in the last tile, an
+    even and an odd number, and a full one.  High blocks run where every SM has one: sequences for that."""
+    import torch
+    from amdmigraphx_b200 import capi
+    sms = torch.cuda.get_device_properties(cuda_device).multi_processor_count
+    batch, heads = (2, 2) if groups == 2 else (-(-sms // tiles), 1)
     for seq in (64 * tiles - 63, 64 * tiles - 31, 64 * tiles):
-        if batch == 2 or tiles <= 3 or seq % 64 == 33:
-            check_attention(cuda_device, batch, seq, 2 if batch == 2 else 1)
+        if groups == 2 or tiles <= 3 or seq % 64 == 33:
+            n = heads * 64
+            x = torch.zeros((batch * seq, 3 * n), dtype=torch.float16, device=cuda_device)
+            names = launched(lambda: capi.attention(x[:, :n], x[:, n:2 * n], x[:, 2 * n:], batch, seq, heads, 0.125))
+            assert len(names) == 1 and "attention_f16_chain_kernelILi%dELi%dEE" % (tiles, groups) in names[0][0], names
+            check_attention(cuda_device, batch, seq, heads)
 
 
 def check_attention(cuda_device, batch, seq, heads):

@@ -5,6 +5,7 @@ fp16 outputs within rtol 2e-2 / atol 1e-2."""
 import numpy as np
 import pytest
 
+from launched import qgemm_form
 from oracle import mgx_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -419,20 +420,21 @@ def test_ragged_rows_take_the_vector_epilogue(cuda_device, M):
     assert (out[0, M:] == 7.0).all() and (q[0, M:] == 9).all()
 
 
-# (on 148 SMs: 256 x 224, 192, 224, 192, 192 with more than eight rows of tiles, 128, 256)
-PAIRS = [(257, 8190, 8208), (700, 4000, 2000), (1000, 8180, 8192), (2300, 4100, 4112), (2500, 1030, 6160), (250, 8200, 8192),
-         (2040, 4090, 4096)]
+# columns of a pair's tile on 148 SMs; the fifth has more than eight rows of tiles
+PAIRS = [(257, 8190, 8208, 224), (700, 4000, 2000, 192), (1000, 8180, 8192, 224), (2300, 4100, 4112, 192), (2500, 1030, 6160, 192),
+         (250, 8200, 8192, 128), (2040, 4090, 4096, 256)]
 
 
-@pytest.mark.parametrize("M,N,K", PAIRS)
-def test_tiles_of_two_ctas_int8_bit_exact(cuda_device, M, N, K):
+@pytest.mark.parametrize("M,N,K,columns", PAIRS)
+def test_tiles_of_two_ctas_int8_bit_exact(cuda_device, M, N, K, columns):
     """Ragged last tiles in M, N and K, several tiles per pair; int32 exact (8-bit products, summed in int64 here)."""
     import torch
     from amdmigraphx_b200 import capi
     rng = np.random.default_rng(M + N + K)
     a, w = _rand_i8(rng, (M, K)), _rand_i8(rng, (N, K))
     out = torch.full((1, M + 8, N), 7, dtype=torch.int32, device=cuda_device)
-    capi.qgemm(_t(a, cuda_device), _t(w, cuda_device), b_layout=capi.B_NK, out=out[:, :M])
+    a_t, w_t = _t(a, cuda_device), _t(w, cuda_device)
+    assert qgemm_form(lambda: capi.qgemm(a_t, w_t, b_layout=capi.B_NK, out=out[:, :M])) == (columns, "pair")
     # 2^14 x 8208 < 2^53: fp64 products of int8 values are exact
     ref = torch.from_numpy(a).to(cuda_device).double() @ torch.from_numpy(w).to(cuda_device).double().T
     assert torch.equal(out[0, :M].double(), ref) and (out[0, M:] == 7).all()
@@ -440,8 +442,8 @@ def test_tiles_of_two_ctas_int8_bit_exact(cuda_device, M, N, K):
 
 
 @pytest.mark.parametrize("kind", ["fp8", "f16"])
-@pytest.mark.parametrize("M,N,K", PAIRS)
-def test_tiles_of_two_ctas_fp(cuda_device, M, N, K, kind):
+@pytest.mark.parametrize("M,N,K,columns", PAIRS)
+def test_tiles_of_two_ctas_fp(cuda_device, M, N, K, columns, kind):
     """Against fp64: the accumulators are fp32 sums of exact products, |error| <= K 2^-24 |a| |b| in any order; the
     bound here is 4e-6 of that product, the half result one step of a half more."""
     import torch
@@ -451,7 +453,9 @@ def test_tiles_of_two_ctas_fp(cuda_device, M, N, K, kind):
     a = torch.randn(M, K, generator=g, device=cuda_device).to(qt)
     w = torch.randn(N, K, generator=g, device=cuda_device).to(qt)
     bias = torch.randn(N, generator=g, device=cuda_device)
-    got = capi.qgemm(a, w, b_layout=capi.B_NK, bias=bias, act="relu", out_dtype=torch.float16).double()
+    out = torch.empty(M, N, dtype=torch.float16, device=cuda_device)
+    assert qgemm_form(lambda: capi.qgemm(a, w, b_layout=capi.B_NK, bias=bias, act="relu", out=out)) == (columns, "pair")
+    got = out.double()
     ref = torch.relu(a.double() @ w.double().T + bias.double())
     mag = a.double().abs() @ w.double().abs().T + bias.double().abs()
     assert ((got - ref).abs() <= 4e-6 * mag + ref.abs() * 2.0 ** -10 + 2.0 ** -24).all()
@@ -477,19 +481,26 @@ def test_tiles_of_two_ctas_residual_and_quantised_result(cuda_device):
     assert (out[0, M:] == 7.0).all() and (q[0, M:] == 9).all()
 
 
-# (K shared by two, four and eight CTAs of a cluster on 148 SMs; ragged rows, columns and shares of K)
-SHARED_K = [(384, 768, 3072), (100, 1000, 4112), (17, 130, 8176), (129, 600, 4800), (500, 1000, 4224), (33, 17, 8992)]
+# CTAs of a cluster that share K on 148 SMs; ragged rows, columns and shares of K.  (fp16 operands of the second have
+# twice the blocks of K, and eight CTAs.)
+SHARED_K = [(384, 768, 3072, 4), (100, 1000, 4112, 4), (17, 130, 8176, 8), (129, 600, 4800, 4), (500, 1000, 4224, 2),
+            (33, 17, 8992, 8)]
 
 
-@pytest.mark.parametrize("M,N,K", SHARED_K)
-def test_shared_k_int8_bit_exact(cuda_device, M, N, K):
+def _tiles_of_64(batch, M, N):
+    return batch * -(-M // 128) * -(-N // 64)
+
+
+@pytest.mark.parametrize("M,N,K,ctas", SHARED_K)
+def test_shared_k_int8_bit_exact(cuda_device, M, N, K, ctas):
     import torch
     from amdmigraphx_b200 import capi
     rng = np.random.default_rng(M + N + K)
     a, w = _rand_i8(rng, (M, K)), _rand_i8(rng, (N, K))
     ref = O.quant_dot_int8(a, w.T)
     out = torch.full((1, M + 8, N), 7, dtype=torch.int32, device=cuda_device)
-    capi.qgemm(_t(a, cuda_device), _t(w, cuda_device), b_layout=capi.B_NK, out=out[:, :M])
+    a_t, w_t = _t(a, cuda_device), _t(w, cuda_device)
+    assert qgemm_form(lambda: capi.qgemm(a_t, w_t, b_layout=capi.B_NK, out=out[:, :M]), _tiles_of_64(1, M, N)) == (64, ctas)
     np.testing.assert_array_equal(out[0, :M].cpu().numpy(), ref)
     assert (out[0, M:] == 7).all()
     scale = rng.uniform(1e-6, 1e-5, size=N).astype(np.float32)
@@ -505,8 +516,8 @@ def test_shared_k_int8_bit_exact(cuda_device, M, N, K):
 
 
 @pytest.mark.parametrize("kind", ["fp8", "f16"])
-@pytest.mark.parametrize("M,N,K", SHARED_K)
-def test_shared_k_fp(cuda_device, M, N, K, kind):
+@pytest.mark.parametrize("M,N,K,ctas", SHARED_K)
+def test_shared_k_fp(cuda_device, M, N, K, ctas, kind):
     """fp32 partial sums added in the order of the shares: the bound of one accumulator holds for their sum."""
     import torch
     from amdmigraphx_b200 import capi
@@ -515,7 +526,41 @@ def test_shared_k_fp(cuda_device, M, N, K, kind):
     a = torch.randn(M, K, generator=g, device=cuda_device).to(qt)
     w = torch.randn(N, K, generator=g, device=cuda_device).to(qt)
     bias = torch.randn(N, generator=g, device=cuda_device)
-    got = capi.qgemm(a, w, b_layout=capi.B_NK, bias=bias, out_dtype=torch.float32).double()
+    out = torch.empty(M, N, device=cuda_device)
+    form = qgemm_form(lambda: capi.qgemm(a, w, b_layout=capi.B_NK, bias=bias, out=out), _tiles_of_64(1, M, N))
+    assert form == (64, 8 if kind == "f16" and (M, N, K) == (100, 1000, 4112) else ctas)
+    got = out.double()
     ref = a.double() @ w.double().T + bias.double()
     mag = a.double().abs() @ w.double().abs().T + bias.double().abs()
     assert ((got - ref).abs() <= 4e-6 * mag).all()
+
+
+@pytest.mark.parametrize("batch,M,N,K,form", [
+    (3, 700, 1000, 4112, (128, "pair")), (4, 257, 2000, 2064, (224, "pair")),
+    (3, 500, 320, 4224, (64, 2)), (3, 100, 200, 4112, (64, 4)), (2, 40, 130, 8208, (64, 8))])
+def test_forms_over_batches_strides_and_results(cuda_device, batch, M, N, K, form):
+    """Several matrices with rows further apart than K, a scale per row, operands in [K,N], and an fp8 result beside
+    the fp32 one, on tiles of two CTAs and with a shared K (148 SMs).  All exact: int32 sums; one product in double
+    and one sum in fp32; a division by a power of two."""
+    import torch
+    from amdmigraphx_b200 import capi
+    rng = np.random.default_rng(batch * M + N + K)
+    a = _t(rng.integers(-128, 128, size=(batch, M, K + 48), dtype=np.int8), cuda_device)[:, :, :K]
+    w = _t(rng.integers(-128, 128, size=(batch, N, K + 16), dtype=np.int8), cuda_device)[:, :, :K]
+    acc = torch.bmm(a.double(), w.double().transpose(1, 2))
+    scale = _t(rng.uniform(1e-6, 1e-5, size=M).astype(np.float32), cuda_device)
+    bias = _t(rng.normal(0, 0.5, size=N).astype(np.float32), cuda_device)
+    out = torch.empty(batch, M, N, dtype=torch.int32, device=cuda_device)
+    assert qgemm_form(lambda: capi.qgemm(a, w, b_layout=capi.B_NK, out=out), _tiles_of_64(batch, M, N)) == form
+    assert torch.equal(out.double(), acc)
+    out.zero_()
+    capi.qgemm(a, w.transpose(1, 2).contiguous(), b_layout=capi.B_KN, out=out)
+    assert torch.equal(out.double(), acc)
+    y = torch.empty(batch, M, N, device=cuda_device)
+    q = torch.empty(batch, M, N, dtype=torch.float8_e4m3fn, device=cuda_device)
+    capi.qgemm(a, w, b_layout=capi.B_NK, scale=scale, scale_mode=capi.SCALE_PER_ROW, bias=bias, out=y, q_out=q, q_scale=0.0078125)
+    want = (acc * scale.double()[None, :, None]).float() + bias
+    assert torch.equal(y, want)
+    fp8 = O.fp8e4m3fn_decode(O.quantizelinear(want.cpu().numpy(), np.array([0.0078125], dtype=np.float32), None, "fp8e4m3fn"))
+    np.testing.assert_array_equal(q.float().cpu().numpy(), fp8)
+    assert capi.device_status() == 0
