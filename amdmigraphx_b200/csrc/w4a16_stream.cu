@@ -51,7 +51,7 @@ struct st_params
     int64_t lda, ldd, N, row_bytes; // row_bytes: K / 2
     int M, groups;                  // groups of 128 k
     int rshift, groups_per_row;     // scale of group g: g >> rshift
-    int scale_vec;                  // scales of a step's groups read together: 4, 2 or 1
+    int scale_vec, zp_vec;          // scales and zero points of a step's groups read together: 4, 2 or 1
     int zp_const;
     int clusters, split, split_log; // CTAs of a cluster
     int tiles_each, tiles_left; // tiles of a cluster; so many clusters have one more
@@ -211,45 +211,70 @@ __global__ void __launch_bounds__(ST_THREADS, 1) w4a16_stream_kernel(const st_pa
     uint32_t zps[(NT * GS + 1) / 2];
     auto load_meta = [&] {
         const int grp = g_lo + GS * (steps - left);
-        auto load     = [&](int i, int j) { // one scale
-            return static_cast<uint32_t>(
-                __half_as_ushort(p.scales[index[i] + (min(grp + j, g_lo + mine - 1) >> p.rshift)]));
-        };
-#pragma unroll
-        for(int i = 0; i < 2 * NT; ++i)
+        const int end = mine - 1 - (grp - g_lo); // the last group of this CTA, from grp on
+        // (grp is a multiple of GS.  A tile's last step may read what belongs to groups beyond it, of this row or the
+        // next: not used.)
+        if(p.rshift > 0)
         {
-            // (a tile's last step may read scales of groups beyond it, of this row or the next: not used)
-            const __half* at = p.scales + index[i] + grp;
-            if(GS == 4 and p.scale_vec == 4)
-            {
-                const uint2 v           = *reinterpret_cast<const uint2*>(at);
-                sc[i * GS / 2]          = v.x;
-                sc[(i * GS + GS - 1) / 2] = v.y;
-            }
-            else if(p.scale_vec >= 2)
-            {
+            // two neighbours share a scale and a zero point
+#pragma unroll
+            for(int i = 0; i < 2 * NT; ++i)
 #pragma unroll
                 for(int j = 0; j < GS; j += 2)
-                    sc[(i * GS + j) / 2] = *reinterpret_cast<const uint32_t*>(at + min(j, (mine - 1 - (grp - g_lo)) & ~1));
-            }
-            else
-            {
+                    sc[(i * GS + j) / 2] =
+                        __half_as_ushort(p.scales[index[i] + ((grp + min(j, end)) >> p.rshift)]) * 0x00010001u;
+        }
+        else
+        {
 #pragma unroll
-                for(int j = 0; j < GS; j += 2)
-                    sc[(i * GS + j) / 2] = load(i, j) | load(i, j + 1) << 16;
+            for(int i = 0; i < 2 * NT; ++i)
+            {
+                const __half* at = p.scales + index[i] + grp;
+                if(GS == 4 and p.scale_vec == 4)
+                {
+                    const uint2 v           = *reinterpret_cast<const uint2*>(at);
+                    sc[i * GS / 2]          = v.x;
+                    sc[(i * GS + GS - 1) / 2] = v.y;
+                }
+                else
+                {
+#pragma unroll
+                    for(int j = 0; j < GS; j += 2)
+                        sc[(i * GS + j) / 2] = p.scale_vec >= 2
+                                                   ? *reinterpret_cast<const uint32_t*>(at + min(j, end & ~1))
+                                                   : static_cast<uint32_t>(__half_as_ushort(at[min(j, end)])) |
+                                                         static_cast<uint32_t>(__half_as_ushort(at[min(j + 1, end)])) << 16;
+                }
             }
         }
         if(has_zp)
         {
-#pragma unroll
-            for(int i = 0; i < (NT * GS + 1) / 2; ++i)
-                zps[i] = 0u;
+            // 16 bits for two groups of a row.  (A byte at a time, and two conversions a row and group: with zero points
+            // 12288 x 4096 at 1 and 16 rows 12.0 and 18.5 us, 4096 x 4096 7.0 and 10.0; so 11.5 and 17.9, 6.7 and 9.7.)
+            uint32_t pair[NT * GS];
 #pragma unroll
             for(int i = 0; i < 2 * NT; ++i)
+            {
+                const uint8_t* at = p.zp + index[i] + (p.rshift > 0 ? 0 : grp);
+                if(GS == 4 and p.rshift == 0 and p.zp_vec == 4)
+                {
+                    const uint32_t v               = *reinterpret_cast<const uint32_t*>(at);
+                    pair[i * GS / 2]               = v & 0xFFFFu;
+                    pair[(i * GS + GS - 1) / 2] = v >> 16;
+                }
+                else
+                {
 #pragma unroll
-                for(int j = 0; j < GS; ++j)
-                    zps[(i * GS + j) / 4] |= static_cast<uint32_t>(p.zp[index[i] + (min(grp + j, g_lo + mine - 1) >> p.rshift)])
-                                             << (8 * ((i * GS + j) & 3));
+                    for(int j = 0; j < GS; j += 2)
+                        pair[(i * GS + j) / 2] =
+                            p.rshift > 0     ? at[(grp + min(j, end)) >> p.rshift] * 0x0101u
+                            : p.zp_vec >= 2 ? *reinterpret_cast<const uint16_t*>(at + min(j, end & ~1))
+                                             : at[min(j, end)] | static_cast<uint32_t>(at[min(j + 1, end)]) << 8;
+                }
+            }
+#pragma unroll
+            for(int i = 0; i < NT * GS; i += 2)
+                zps[i / 2] = pair[i] | (i + 1 < NT * GS ? pair[i + 1] << 16 : 0u);
         }
     };
     meta_rows();
@@ -297,14 +322,10 @@ __global__ void __launch_bounds__(ST_THREADS, 1) w4a16_stream_kernel(const st_pa
     // ---- steps
     uint32_t magic;
     asm volatile("mov.b32 %0, 0x64006400;" : "=r"(magic));
-    auto z_pairs = [](int z, __half2& z0, __half2& z1) {
-        z0 = __half2half2(__int2half_rn(-1024 - z));
-        z1 = __half2half2(__int2half_rn(-64 - z));
-    };
     __half2 z0[2 * NT], z1[2 * NT]; // of the rows
 #pragma unroll
     for(int i = 0; i < 2 * NT; ++i)
-        z_pairs(p.zp_const, z0[i], z1[i]);
+        z0[i] = __half2half2(__int2half_rn(-1024 - p.zp_const)), z1[i] = __half2half2(__int2half_rn(-64 - p.zp_const));
     // rows beyond M read one that exists; their columns are not stored
     const uint8_t* act_row[MT];
     auto act_rows = [&] {
@@ -359,8 +380,11 @@ __global__ void __launch_bounds__(ST_THREADS, 1) w4a16_stream_kernel(const st_pa
 #pragma unroll
                 for(int i = 0; i < 2 * NT; ++i)
                 {
-                    const int e = i * GS + j;
-                    z_pairs(z[e / 4] >> (8 * (e & 3)) & 0xFFu, z0[i], z1[i]);
+                    // 0xE400 | z is -(1024 + z); 960 more is -(64 + z), exactly
+                    const int e      = i * GS + j;
+                    const uint32_t b = __byte_perm(z[e / 4], 0xE4E4E4E4u, 0x4040u | (e & 3) * 0x0101u);
+                    z0[i]            = *reinterpret_cast<const __half2*>(&b);
+                    z1[i]            = __hadd2(z0[i], __float2half2_rn(960.0f));
                 }
             }
 #pragma unroll
@@ -621,11 +645,15 @@ int w4a16_stream_launch(const mgx_w4_desc& d, const void* A, const void* Bp, con
     for(p.rshift = 0; (ST_GROUP_K << p.rshift) < d.group; ++p.rshift)
         ;
     p.zp_const = d.zp_const;
-    // scales of four or two groups are one aligned access
-    const auto align = [&](int v) {
-        return p.rshift == 0 and p.groups_per_row % v == 0 and reinterpret_cast<uintptr_t>(scales) % (2 * v) == 0;
+    // scales (2 bytes) and zero points (1 byte) of four or two groups are one aligned access
+    const auto together = [&](const void* at, int bytes) {
+        for(int v : {4, 2})
+            if(p.groups_per_row % v == 0 and reinterpret_cast<uintptr_t>(at) % (bytes * v) == 0)
+                return v;
+        return 1;
     };
-    p.scale_vec = align(4) ? 4 : (align(2) ? 2 : 1);
+    p.scale_vec = together(scales, 2);
+    p.zp_vec    = together(zp, 1);
     return d.M <= 8 ? launch_best<st_form<1, 1, 4, 2>, st_form<1, 1, 2, 4>, st_form<1, 1, 2, 2>>(p, stream)
                     : launch_best<st_form<2, 2, 2, 2>, st_form<2, 1, 2, 4>, st_form<2, 1, 2, 2>>(p, stream);
 }
