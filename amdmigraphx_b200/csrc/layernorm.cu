@@ -52,14 +52,16 @@ struct ln_params
 // T: float or __half.  NV: 16-byte vectors per thread.  WPR: warps per row - 1 (a warp per row, a
 // thread owns vectors lane, lane + 32, ...) or 8 (a block per row: few, long rows, e.g. the single
 // token of a decode step, where one warp per row would leave a 4096-element row to 32 threads).
-template <class T, int NV, int WPR>
+// EARLY: gamma and beta come with the row, and what follows may start when they have been requested: for rows that are
+// few enough to be there all at once.
+template <class T, int NV, int WPR, bool EARLY = false>
 __global__ void __launch_bounds__(256) layernorm_kernel(const ln_params p)
 {
     constexpr int VE  = 16 / sizeof(T); // elements per vector
     constexpr int TPR = 32 * WPR;       // threads per row
     __shared__ float red[2][8];
-    // Chained to its neighbours; what follows sets itself up (an int4 linear: requests its weights) while this runs
-    // (see launch_rows) - once this row's operands are requested, which would else wait behind the weights.
+    // (EARLY: what follows sets itself up, an int4 linear requests its weights, while this runs (see launch_rows) - once
+    // this row's operands are requested, which would else wait behind the weights.)
     grid_dependency_wait();
     const int lane    = WPR == 1 ? (threadIdx.x & 31) : threadIdx.x;
     const int64_t row = WPR == 1 ? static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)
@@ -87,8 +89,6 @@ __global__ void __launch_bounds__(256) layernorm_kernel(const ln_params p)
     const T* xr    = static_cast<const T*>(p.x) + row * p.ldx;
     float v[NV][VE];
     float sum = 0.0f;
-    // gamma and beta come with the row where there are registers for them
-    constexpr bool EARLY = NV <= 4;
     const T* g = static_cast<const T*>(p.gamma);
     const T* b = static_cast<const T*>(p.beta);
     uint4 gw[EARLY ? NV : 1], bw[EARLY ? NV : 1];
@@ -138,8 +138,9 @@ __global__ void __launch_bounds__(256) layernorm_kernel(const ln_params p)
                 v[i][j] = 0.0f;
         }
     }
-    if(p.q == nullptr)
-        grid_launch_dependents();
+    if constexpr(EARLY)
+        if(p.q == nullptr)
+            grid_launch_dependents();
     float mean = 0.0f;
     if(not p.rms)
         mean = ln_round<T>(row_sum(sum, 0) * p.inv_n);
@@ -288,9 +289,9 @@ __global__ void __launch_bounds__(256) layernorm_kernel(const ln_params p)
 
 // 256 threads a block, launched programmatically: a layer's norm starts 1 to 2 us earlier behind a GEMM (encoder layer
 // of 985 rows, launched one by one, 63.0 -> 58.5 us; of 3072 rows in a graph 105.4 -> 104.8).  What follows may start
-// early too unless the result is quantised: an int8 result may be packed weights (ptx.cuh).  An int4 decode linear
-// behind an RMSNorm then begins 2 us earlier (one row, norm and linear back to back: 4096 x 4096 10.2 -> 8.0 us,
-// 12288 x 4096 12.3 -> 10.4).
+// early too where the form is EARLY, unless the result is quantised: an int8 result may be packed weights (ptx.cuh).  An
+// int4 decode linear behind an RMSNorm then begins 2 us earlier (one row, norm and linear back to back: 4096 x 4096
+// 10.2 -> 8.0 us, 12288 x 4096 12.3 -> 10.4).
 static int launch_rows(void (*kernel)(ln_params), dim3 grid, const ln_params& p, cudaStream_t stream)
 {
     return launch_dependent(kernel, grid, dim3(256), 0, stream, p);
@@ -311,11 +312,15 @@ static int launch_layernorm(const ln_params& p, cudaStream_t stream)
         const int nv = (nvec + 255) / 256;
         const dim3 grid(static_cast<unsigned>(p.rows));
         if(nv <= 1)
-            return launch_rows(layernorm_kernel<T, 1, 8>, grid, p, stream);
+            return launch_rows(layernorm_kernel<T, 1, 8, true>, grid, p, stream);
         if(nv <= 2)
-            return launch_rows(layernorm_kernel<T, 2, 8>, grid, p, stream);
+            return launch_rows(layernorm_kernel<T, 2, 8, true>, grid, p, stream);
+        // (the registers of EARLY cost where a block has successors on its SM.  8192 halves a row, without and with: 512
+        // rows 6.5 / 5.6 us, 1024 9.4 / 10.4, 8192 56 / 71.  The forms above run for up to eight rows an SM: 1024 rows of
+        // 4096 5.3 / 5.0, of 768 3.9 / 3.2; the warp forms below for more: 8192 rows of 1024 12.9 / 14.6)
         if(nv <= 4)
-            return launch_rows(layernorm_kernel<T, 4, 8>, grid, p, stream);
+            return launch_rows(p.rows <= 4 * device_sm_count() ? layernorm_kernel<T, 4, 8, true> : layernorm_kernel<T, 4, 8>,
+                               grid, p, stream);
         if(nv <= 8)
             return launch_rows(layernorm_kernel<T, 8, 8>, grid, p, stream);
         return MGX_E_UNSUPPORTED;

@@ -60,6 +60,29 @@ def test_layernorm_only_quantised_output_and_no_affine(cuda_device):
     np.testing.assert_array_equal(dq.cpu().numpy().view(np.uint16), np.asarray(dq_ref, dtype=np.float16).view(np.uint16))
 
 
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("cols,dtype", [(8192, "float16"), (4096, "float32"), (6152, "float16")])
+def test_layernorm_of_long_rows_few_and_many(cuda_device, cols, dtype, rms):
+    """Up to four rows an SM gamma and beta are fetched with the row, beyond that behind it: the same bits."""
+    import torch
+    from amdmigraphx_b200 import capi
+    few = 4 * torch.cuda.get_device_properties(cuda_device).multi_processor_count
+    dt = getattr(torch, dtype)
+    g = torch.Generator(device=cuda_device).manual_seed(cols)
+    x, gamma, beta = (torch.randn(s, generator=g, device=cuda_device).to(dt) for s in ((few + 1, cols), (cols,), (cols,)))
+    beta = None if rms else beta
+    names = [launched(lambda: capi.layernorm(x[:n], gamma, beta, 1e-5, rms=rms))[0][0] for n in (few, few + 1)]
+    assert names[0] != names[1]
+    a, b = (capi.layernorm(x[:n], gamma, beta, 1e-5, rms=rms)[0] for n in (few, few + 1))
+    assert torch.equal(a, b[:few])
+    v = x[few].double()
+    v = v if rms else v - v.mean()
+    ref = v / (v.square().mean() + 1e-5).sqrt() * gamma.double() + (0.0 if rms else beta.double())
+    # every operator of the chain stores its type: eight roundings of 2^-10 of the row's terms
+    step = 2.0 ** (-10 if dtype == "float16" else -20)
+    assert ((b[few].double() - ref).abs() <= 8 * step * (ref.abs() + gamma.double().abs() + 1)).all()
+
+
 @pytest.mark.parametrize("batch,seq,heads", [(1, 384, 12), (2, 200, 4), (3, 64, 2), (1, 77, 1), (8, 384, 12),
                                              (1, 1024, 2), (1, 1100, 2)])
 def test_attention_matches_chain(cuda_device, batch, seq, heads):
