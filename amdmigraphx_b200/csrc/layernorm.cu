@@ -315,14 +315,15 @@ static int launch_layernorm(const ln_params& p, cudaStream_t stream)
             return launch_rows(layernorm_kernel<T, 1, 8, true>, grid, p, stream);
         if(nv <= 2)
             return launch_rows(layernorm_kernel<T, 2, 8, true>, grid, p, stream);
-        // (the registers of EARLY cost where a block has successors on its SM.  8192 halves a row, without and with: 512
+        // (The registers of EARLY cost where a block has successors on its SM.  8192 halves a row, without and with: 512
         // rows 6.5 / 5.6 us, 1024 9.4 / 10.4, 8192 56 / 71.  The forms above run for up to eight rows an SM: 1024 rows of
         // 4096 5.3 / 5.0, of 768 3.9 / 3.2; the warp forms below for more: 8192 rows of 1024 12.9 / 14.6)
         if(nv <= 4)
             return launch_rows(p.rows <= 4 * device_sm_count() ? layernorm_kernel<T, 4, 8, true> : layernorm_kernel<T, 4, 8>,
                                grid, p, stream);
         if(nv <= 8)
-            return launch_rows(layernorm_kernel<T, 8, 8>, grid, p, stream);
+            return launch_rows(p.rows <= device_sm_count() ? layernorm_kernel<T, 8, 8, true> : layernorm_kernel<T, 8, 8>, grid,
+                               p, stream);
         return MGX_E_UNSUPPORTED;
     }
     const int nv    = (nvec + 31) / 32;

@@ -61,12 +61,13 @@ def test_layernorm_only_quantised_output_and_no_affine(cuda_device):
 
 
 @pytest.mark.parametrize("rms", [False, True])
-@pytest.mark.parametrize("cols,dtype", [(8192, "float16"), (4096, "float32"), (6152, "float16")])
-def test_layernorm_of_long_rows_few_and_many(cuda_device, cols, dtype, rms):
-    """Up to four rows an SM gamma and beta are fetched with the row, beyond that behind it: the same bits."""
+@pytest.mark.parametrize("cols,dtype,rows", [(8192, "float16", 4), (4096, "float32", 4), (6152, "float16", 4),
+                                             (16384, "float16", 1), (8196, "float32", 1)])
+def test_layernorm_of_long_rows_few_and_many(cuda_device, cols, dtype, rows, rms):
+    """Up to `rows` rows an SM gamma and beta are fetched with the row, beyond that behind it: the same bits."""
     import torch
     from amdmigraphx_b200 import capi
-    few = 4 * torch.cuda.get_device_properties(cuda_device).multi_processor_count
+    few = rows * torch.cuda.get_device_properties(cuda_device).multi_processor_count
     dt = getattr(torch, dtype)
     g = torch.Generator(device=cuda_device).manual_seed(cols)
     x, gamma, beta = (torch.randn(s, generator=g, device=cuda_device).to(dt) for s in ((few + 1, cols), (cols,), (cols,)))
