@@ -199,12 +199,13 @@ __global__ void __launch_bounds__(GD_THREADS + 32, 2)
             ++xch;
         };
         // what the CTAs of the cluster hold at `at`, added in their order, or the largest: all under way together (one
-        // after another 0.2 us each)
+        // after another 0.2 us each; eight reads for two CTAs: 32 heads, 128 positions 6.1 -> 6.4 us)
         auto of_cluster = [&](const float* at, bool largest) {
             float v[GD_MAX_SPLIT];
 #pragma unroll
             for(int r = 0; r < GD_MAX_SPLIT; ++r)
-                v[r] = __uint_as_float(cluster_load(at, min(r, p.split - 1)));
+                if(r < p.split)
+                    v[r] = __uint_as_float(cluster_load(at, r));
             float x = v[0];
 #pragma unroll
             for(int r = 1; r < GD_MAX_SPLIT; ++r)
