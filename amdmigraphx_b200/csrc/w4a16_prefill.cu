@@ -497,14 +497,22 @@ int max_clusters(int split)
 void pf_plan(const mgx_w4_desc& d, pf_params& p)
 {
     const int64_t tiles_n = ceil_div(d.N, PF_ROWS), groups = d.K / PF_GROUP_K, sms = device_sm_count();
-    double best = 0.0;
-    for(int64_t tiles_m = ceil_div(d.M, PF_MAX_TOKENS); tiles_m <= ceil_div(d.M, 64); ++tiles_m)
+    double best  = 0.0;
+    int64_t last = 0;
+    const int clusters[3] = {max_clusters(2), max_clusters(4), max_clusters(8)};
+    // Of the numbers of tiles with the same rows in a tile the smallest is the best: one candidate for every multiple of
+    // 16 rows, whatever M is.
+    for(int rows = PF_MAX_TOKENS; rows > 0 and ceil_div(d.M, rows) <= ceil_div(d.M, 64); rows -= 16)
     {
+        const int64_t tiles_m = ceil_div(d.M, rows);
+        if(tiles_m == last)
+            continue;
+        last                = tiles_m;
         const int tokens    = static_cast<int>(ceil_div(ceil_div(d.M, tiles_m), 16) * 16);
         const int64_t tiles = tiles_n * tiles_m;
         int split           = 1;
-        for(int s = 2; s <= PF_MAX_SPLIT and groups >= 4 * s and tiles <= max_clusters(s); s *= 2)
-            split = s;
+        for(int i = 0; i < 3 and groups >= 8 << i and tiles <= clusters[i]; ++i)
+            split = 2 << i;
         const double group = std::max({4.0 * tokens, pf_stage(tokens) / 62.0, 560.0}) + 100.0;
         const double waves = split > 1 ? 1.0 : static_cast<double>(ceil_div(tiles, sms));
         const double alone = 12.0 * tokens; // the last tile's epilogue, and every one's with two accumulators
