@@ -23,7 +23,10 @@ CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "lib")
 OBJ = os.path.join(PKG, "build")
 
-KERNEL_SOURCES = ["runtime.cu", "quantize.cu", "qgemm.cu", "qgemm_pair_f8.cu", "qgemm_pair_i8.cu", "qgemm_f8.cu", "qgemm_i8.cu", "qgemm_pair_f16.cu", "qgemm_f16.cu", "qgemm_split.cu", "qgemv.cu", "pointwise.cu", "reduce.cu", "layernorm.cu", "attention.cu", "kvcache.cu", "gqa_decode.cu", "gather.cu", "w4a16.cu", "w4a16_stream.cu", "w4a16_tc.cu", "w4a16_prefill.cu", "comm.cu"]
+KERNEL_SOURCES = ["runtime.cu", "quantize.cu", "qgemm.cu", "qgemm_split.cu", "qgemv.cu", "pointwise.cu", "reduce.cu", "layernorm.cu", "attention.cu", "kvcache.cu", "gqa_decode.cu", "gather.cu", "w4a16.cu", "w4a16_stream.cu", "w4a16_tc.cu", "w4a16_prefill.cu", "comm.cu"]
+# qgemm_form.cu is compiled once for every form of the kernel: operand type, kind of tile, its columns
+QGEMM_FORMS = [(t, k, bn) for t in ("i8", "f8", "f16")
+               for k, widths in (("one", (64, 128, 256)), ("pair", (128, 192, 224, 256)), ("split", (64,))) for bn in widths]
 KERNEL_LIB = os.path.join(LIB, "libmgx_cuda_kernels.so")
 TORCH_OPS = os.path.join(LIB, "mgx_torch_ops.so")
 
@@ -53,11 +56,20 @@ def _headers():
     return hs
 
 
+def _jobs():
+    """(source, object, definitions) of the kernel library, the longest to compile first."""
+    forms = sorted(QGEMM_FORMS, key=lambda f: (f[1] == "one", -f[2]))
+    jobs = [(os.path.join(CSRC, "qgemm_form.cu"), os.path.join(OBJ, f"qgemm_{t}_{k}_{bn}.o"),
+             [f"-DMGX_FORM={t}_{k}_{bn}", f"-DMGX_FORM_TYPE={('i8', 'f8', 'f16').index(t)}",
+              f"-DMGX_FORM_KIND=QGEMM_{k.upper()}", f"-DMGX_FORM_BN={bn}"]) for t, k, bn in forms]
+    return jobs + [(os.path.join(CSRC, s), os.path.join(OBJ, s[:-3] + ".o"), []) for s in KERNEL_SOURCES]
+
+
 def _compile(args):
-    src, obj, verbose, force = args
+    src, obj, defines, verbose, force = args
     if not force and not _newer(obj, [src] + _headers()):
         return src, 0, ""
-    cmd = [nvcc_path(), "-c", src, "-o", obj] + NVCC_FLAGS
+    cmd = [nvcc_path(), "-c", src, "-o", obj] + defines + NVCC_FLAGS
     if verbose:
         cmd += ["-Xptxas", "-v"]
     r = subprocess.run(cmd, capture_output=True, text=True)
@@ -67,9 +79,8 @@ def _compile(args):
 def build_kernels(verbose=False, force=False):
     os.makedirs(LIB, exist_ok=True)
     os.makedirs(OBJ, exist_ok=True)
-    jobs = [(os.path.join(CSRC, s), os.path.join(OBJ, s[:-3] + ".o"), verbose, force)
-            for s in KERNEL_SOURCES]
-    with cf.ThreadPoolExecutor(len(jobs)) as ex:
+    jobs = [j + (verbose, force) for j in _jobs()]
+    with cf.ThreadPoolExecutor(2 * (os.cpu_count() or 8)) as ex:
         for src, rc, out in ex.map(_compile, jobs):
             if verbose and out:
                 print(out)

@@ -188,18 +188,21 @@ extern "C" int mgx_cuda_qgemm_ex(const mgx_qgemm_desc* d, const void* A, const v
         return qgemv_launch(*d, A, Bk, D, scale, bias, ldb, stream);
     const qgemm_operands o{A, Bk, D, scale, bias, residual, ldb, stride_b};
     const tile_choice tile = pick_tile(*d);
-    if(tile.split > 1)
-        return qgemm_split_launch(tile.split, *d, o, qo, stream);
-    const auto launch = d->ab_type == MGX_I8 ? (tile.pair ? qgemm_pair_i8_launch : qgemm_i8_launch)
-                        : f16                ? (tile.pair ? qgemm_pair_f16_launch : qgemm_f16_launch)
-                                             : (tile.pair ? qgemm_pair_f8_launch : qgemm_f8_launch);
-    return launch(tile.bn, *d, o, qo, stream);
+    const qgemm_kind kind  = tile.split > 1 ? QGEMM_SPLIT : (tile.pair ? QGEMM_PAIR : QGEMM_ONE);
+#define MGX_QGEMM_LAUNCH(NAME, TYPE, KIND, BN)                          \
+    if(d->ab_type == TYPE and kind == KIND and tile.bn == BN)           \
+        return qgemm_launch_##NAME(*d, o, qo, tile.split, stream);
+    MGX_QGEMM_FORMS(MGX_QGEMM_LAUNCH)
+#undef MGX_QGEMM_LAUNCH
+    return MGX_E_UNSUPPORTED;
 }
 
 int mgx::qgemm_status(unsigned int* out)
 {
     *out = 0;
-    for(auto f : {qgemm_i8_status, qgemm_f8_status, qgemm_f16_status, qgemm_pair_i8_status, qgemm_pair_f8_status, qgemm_pair_f16_status, qgemm_split_status})
+#define MGX_QGEMM_STATUS(NAME, TYPE, KIND, BN) qgemm_status_##NAME,
+    for(auto f : {MGX_QGEMM_FORMS(MGX_QGEMM_STATUS)})
+#undef MGX_QGEMM_STATUS
     {
         unsigned int v = 0;
         const int rc   = f(&v);

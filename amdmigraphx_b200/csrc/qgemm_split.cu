@@ -1,17 +1,8 @@
-// quant_dot kernels: tiles of 128 x 64 whose K a cluster shares.
+// quant_dot with a shared K: how many clusters run at once.
 #include "qgemm_kernel.cuh"
 #include <mutex>
 
 namespace mgx {
-
-int qgemm_split_launch(int split, const mgx_qgemm_desc& d, const qgemm_operands& o, const qout_args& qo, cudaStream_t stream)
-{
-    if(d.ab_type == MGX_I8)
-        return dispatch_out<64, true, false, false, true>(d, o, qo, stream, split);
-    if(d.ab_type == MGX_F16)
-        return dispatch_out<64, false, true, false, true>(d, o, qo, stream, split);
-    return dispatch_out<64, false, false, false, true>(d, o, qo, stream, split);
-}
 
 // Stands in for the kernels in the question how many clusters fit: what limits them is the block and its shared memory,
 // the same for all, and to ask for one of them would load its code.
@@ -49,7 +40,5 @@ int qgemm_split_clusters(int split)
     }
     return n;
 }
-
-int qgemm_split_status(unsigned int* out) { return read_and_clear_status(out); }
 
 } // namespace mgx
