@@ -52,7 +52,7 @@ int w4a16_prefill_launch(const mgx_w4_desc& d, const void* A, const void* Bp, co
 
 // int4 decode path for all but the largest matrices (w4a16_stream.cu); _launch gives MGX_E_UNSUPPORTED where the
 // activations do not fit in shared memory, which they do where _fits says so
-bool w4a16_stream_preferred(const mgx_w4_desc& d);
+bool w4a16_stream_preferred(const mgx_w4_desc& d, bool has_zp);
 bool w4a16_stream_fits(const mgx_w4_desc& d);
 int w4a16_stream_launch(const mgx_w4_desc& d, const void* A, const void* Bp, const void* scales, const void* zp, void* D,
                         cudaStream_t stream);

@@ -669,7 +669,7 @@ extern "C" int mgx_cuda_w4a16_gemv(const mgx_w4_desc* d, const void* A, const vo
         const size_t shift = workspace == nullptr ? 0 : (256 - (addr & 255u)) & 255u;
         if(workspace == nullptr or workspace_bytes < shift)
             return MGX_E_WORKSPACE;
-        if(w4a16_stream_preferred(*d))
+        if(w4a16_stream_preferred(*d, zp != nullptr))
         {
             rc = w4a16_stream_launch(*d, A, Bp, scales, zp, D, stream);
             if(rc != MGX_E_UNSUPPORTED) // (no room for the activations)

@@ -611,19 +611,20 @@ int launch_best(const st_params& p, cudaStream_t stream)
 
 static int64_t kb32(const mgx_w4_desc& d) { return ceil_div(d.N, 128) * ceil_div(d.K, 512); }
 
-// Where it is the faster of the two decode kernels, by 32 KB of packed weights per SM.  Up to 4 rows and above 8: up to 7
-// (linears back to back, us, here and w4a16_tc.cu: 4 rows, 8192 x 8192 (6.9) 12.5 and 13.1, with zero points 13.6 and 13.7,
-// 6144 x 11008 (7.1) 12.3 and 12.4, 14.0 and 13.2, 6144 x 14336 (9.1) 15.7 and 15.2, 18.6 and 14.9; 16 rows, 8192 x 8192
-// 17.1 and 18.3, 6144 x 11008 20.4 and 19.1; a norm and 22016 x 4096 (9.3) at 1 row 14.5 and 14.2, at 4 15.2 and 15.7).
+// Where it is the faster of the two decode kernels, by 32 KB of packed weights per SM.  Above 8 rows, and with zero points
+// up to 4: up to 7 (linears back to back, us, here and w4a16_tc.cu: 16 rows, 8192 x 8192 (6.9) 17.1 and 18.3, 6144 x 11008
+// (7.1) 20.4 and 19.1; 4 rows with zero points, the same two 13.6 and 13.7, 14.0 and 13.2, 6144 x 14336 (9.1) 18.6 and
+// 14.9).  Up to 4 rows without: up to 10 (6144 x 11008 12.3 and 12.4, 6144 x 14336 15.7 and 15.2, a norm and 22016 x 4096
+// (9.3) at 4 rows 15.2 and 15.7; in a decoder layer the second kernel's launch costs 2 us more, 64.2 and 66.1).
 // 5 to 8 rows: everywhere (57344 x 8192 (48) 59 and 63), but for large matrices of so long a K that only an eighth of the
 // activations fits beside the large rings, whose clusters leave SMs without one (8 rows, 8192 x 20480 (17) 24.5 and 27.8,
 // 4096 x 28672 (12) 20.3 and 23.5, 6144 x 28672 (18) 30.7 and 29.2, 8192 x 28672 (24) 38.9 and 35.5; 5 rows 31.2 and 35.2).
-bool w4a16_stream_preferred(const mgx_w4_desc& d)
+bool w4a16_stream_preferred(const mgx_w4_desc& d, bool has_zp)
 {
     const int64_t sms = device_sm_count();
     if(d.M > 4 and d.M <= 8)
         return d.M * d.K <= 168 * 1000 or kb32(d) <= 16 * sms;
-    return kb32(d) <= 7 * sms;
+    return kb32(d) <= (d.M <= 4 and not has_zp ? 10 : 7) * sms;
 }
 
 // Activations of an eighth of K beside the smallest rings and the sums of a few tiles.
