@@ -317,7 +317,7 @@ static int launch_layernorm(const ln_params& p, cudaStream_t stream)
             return launch_rows(layernorm_kernel<T, 2, 8, true>, grid, p, stream);
         // (The registers of EARLY cost where a block has successors on its SM.  8192 halves a row, without and with: 512
         // rows 6.5 / 5.6 us, 1024 9.4 / 10.4, 8192 56 / 71.  The forms above run for up to eight rows an SM: 1024 rows of
-        // 4096 5.3 / 5.0, of 768 3.9 / 3.2; the warp forms below for more: 8192 rows of 1024 12.9 / 14.6)
+        // 4096 5.3 / 5.0, of 768 3.9 / 3.2.)
         if(nv <= 4)
             return launch_rows(p.rows <= 4 * device_sm_count() ? layernorm_kernel<T, 4, 8, true> : layernorm_kernel<T, 4, 8>,
                                grid, p, stream);
@@ -329,14 +329,18 @@ static int launch_layernorm(const ln_params& p, cudaStream_t stream)
     const int nv    = (nvec + 31) / 32;
     const int warps = 8;
     const dim3 grid(static_cast<unsigned>((p.rows + warps - 1) / warps));
+    // (EARLY here: behind a GEMM, whose result is in L2, gamma and beta are what a row waits for.  Encoder layers without
+    // and with, us: 1536 and 3072 rows of 768 65.8 / 63.7 and 96.6 / 94.4, 6144 167.8 / 166.8; of 1024, a vector more,
+    // 2304 rows 112.3 / 108.9, 3072 154.7 / 157.5, 6144 249.6 / 251.7.  By itself, 8192 rows of 768 10.0 / 10.7.)
+    const bool early = p.rows <= (nv <= 3 ? 48 : 16) * device_sm_count();
     if(nv <= 1)
-        return launch_rows(layernorm_kernel<T, 1, 1>, grid, p, stream);
+        return launch_rows(early ? layernorm_kernel<T, 1, 1, true> : layernorm_kernel<T, 1, 1>, grid, p, stream);
     if(nv <= 2)
-        return launch_rows(layernorm_kernel<T, 2, 1>, grid, p, stream);
+        return launch_rows(early ? layernorm_kernel<T, 2, 1, true> : layernorm_kernel<T, 2, 1>, grid, p, stream);
     if(nv <= 3)
-        return launch_rows(layernorm_kernel<T, 3, 1>, grid, p, stream);
+        return launch_rows(early ? layernorm_kernel<T, 3, 1, true> : layernorm_kernel<T, 3, 1>, grid, p, stream);
     if(nv <= 4)
-        return launch_rows(layernorm_kernel<T, 4, 1>, grid, p, stream);
+        return launch_rows(early ? layernorm_kernel<T, 4, 1, true> : layernorm_kernel<T, 4, 1>, grid, p, stream);
     if(nv <= 6)
         return launch_rows(layernorm_kernel<T, 6, 1>, grid, p, stream);
     if(nv <= 8)

@@ -62,8 +62,9 @@ def test_layernorm_only_quantised_output_and_no_affine(cuda_device):
 
 @pytest.mark.parametrize("rms", [False, True])
 @pytest.mark.parametrize("cols,dtype,rows", [(8192, "float16", 4), (4096, "float32", 4), (6152, "float16", 4),
-                                             (16384, "float16", 1), (8192, "float32", 1)])
-def test_layernorm_of_long_rows_few_and_many(cuda_device, cols, dtype, rows, rms):
+                                             (16384, "float16", 1), (8192, "float32", 1), (768, "float16", 48),
+                                             (200, "float16", 48), (384, "float32", 48), (1024, "float16", 16)])
+def test_layernorm_of_few_and_many_rows(cuda_device, cols, dtype, rows, rms):
     """Up to `rows` rows an SM gamma and beta are fetched with the row, beyond that behind it: the same bits."""
     import torch
     from amdmigraphx_b200 import capi
