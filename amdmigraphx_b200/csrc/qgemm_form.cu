@@ -1,6 +1,7 @@
 // One form of the quant_dot kernel: MGX_FORM of qgemm_host.cuh's list, given on the command line with its operand type
 // (MGX_FORM_TYPE 0: int8, 1: fp8, 2: fp16), kind (MGX_FORM_KIND) and columns (MGX_FORM_BN).  The first launch of a kernel
-// loads its translation unit, 3.5 ms a MB: with a type's forms in one unit the first tile of a pair cost 16 to 22 ms.
+// loads its translation unit: with a type's forms in one unit the first tile of one CTA cost 16 ms, of a pair 16 to 22, a
+// shared K 12; so 2 to 3 ms each.
 #include "qgemm_kernel.cuh"
 #include <atomic>
 
