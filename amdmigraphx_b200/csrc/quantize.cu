@@ -564,14 +564,20 @@ __global__ void __launch_bounds__(256)
 
 // The same with 16-byte accesses: 64 x 64 elements a block, rows of 72 in shared memory so that the eight elements a
 // thread gathers down a column lie in different banks from its neighbours'.  A prompt's values (32 x 512 x 128, 8 MB
-// moved) 5.6 us an element at a time, 4.6 so.  Launched plainly, as the one above: the GEMM behind it takes whole SMs, and
-// where it could start early it took them from blocks still to come (softmax and dot, 32 x 512 x 512 by 32 x 512 x 128
-// 26.4 us, plainly 21.8; 8 x 1024 x 1024 x 128 17.5 and 13.9).
+// moved) 5.6 us an element at a time, 4.6 so.
+// EARLY: launched programmatically, what follows may start early.  For rows as short as a head's (up to 128), the values
+// of a prompt's attention: a layer of 512 tokens 268.8 us, launched plainly 272.2, of 1000 536 and 567 - though not for
+// such dots directly behind one another (32 x 512 x 128 x 512 14.1 and 12.2 us).  For longer rows plainly: the GEMM behind
+// it takes whole SMs, from blocks still to come (8 x 1024 x 1024 x 128 17.5 us, plainly 13.9, 32 x 512 x 512 x 128 17.6 and
+// 15.4).
+template <bool EARLY>
 __global__ void __launch_bounds__(256)
-    transpose_16bit_vec_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ dst, int64_t rows, int64_t cols,
+    transpose_16bit_vec_kernel(const uint16_t* src, uint16_t* dst, int64_t rows, int64_t cols,
                                int64_t ld_dst)
 {
     __shared__ __align__(16) uint16_t tile[64][72];
+    if constexpr(EARLY)
+        grid_dependency_wait();
     const uint16_t* s = src + blockIdx.z * rows * cols;
     uint16_t* d       = dst + blockIdx.z * cols * ld_dst;
     const int64_t r0 = static_cast<int64_t>(blockIdx.y) * 64, c0 = static_cast<int64_t>(blockIdx.x) * 64;
@@ -582,6 +588,8 @@ __global__ void __launch_bounds__(256)
         if(r0 + rr < rows and c0 + cc < cols)
             *reinterpret_cast<uint4*>(&tile[rr][cc]) = *reinterpret_cast<const uint4*>(s + (r0 + rr) * cols + c0 + cc);
     }
+    if constexpr(EARLY)
+        grid_launch_dependents();
     __syncthreads();
 #pragma unroll
     for(int i = 0; i < 2; ++i)
@@ -614,8 +622,11 @@ int transpose_16bit_ld(const void* src, void* dst, int64_t rows, int64_t cols, i
     if(cols % 8 == 0 and ld_dst % 8 == 0 and (reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) % 16 == 0)
     {
         const dim3 vgrid(static_cast<unsigned>(ceil_div(cols, 64)), static_cast<unsigned>(ceil_div(rows, 64)), static_cast<unsigned>(batch));
-        transpose_16bit_vec_kernel<<<vgrid, 256, 0, stream>>>(static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), rows,
-                                                              cols, ld_dst);
+        const auto* in = static_cast<const uint16_t*>(src);
+        auto* out      = static_cast<uint16_t*>(dst);
+        if(cols <= 128)
+            return launch_dependent(transpose_16bit_vec_kernel<true>, vgrid, dim3(256), 0, stream, in, out, rows, cols, ld_dst);
+        transpose_16bit_vec_kernel<false><<<vgrid, 256, 0, stream>>>(in, out, rows, cols, ld_dst);
         return static_cast<int>(cudaGetLastError());
     }
     dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy), static_cast<unsigned>(batch));
